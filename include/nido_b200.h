@@ -210,13 +210,12 @@ int nido_dump_partition(nido_graph g, const char* path, const int64_t* new_order
  * `stream` (a cudaStream_t, NULL for the legacy default stream), without a
  * host synchronisation.  The reduction follows the reference's order, so Q
  * matches nido_compute_modularity bit for bit on integer weights.
- * Scratch: a fixed 4 MiB array (524,280 FP64 group partials, the
- * reference's own maximum) inside the library, held by every GPU that loads
- * it until exit; it covers any nv up to the limit of 2^31-2 vertices, and
- * larger nv is rejected with NIDO_E_TOO_LARGE.  The first call on a device
- * looks up the array's device address (cudaGetSymbolAddress), so make that
- * first call before any stream capture.  All calls on a device share the
- * array: calls that overlap on the GPU race and return wrong values. */
+ * Scratch: fixed 6 MiB arrays (524,280 FP64 group partials, the
+ * reference's own maximum, and the sums of edge chunks) inside the library,
+ * held by every GPU that loads it until exit; they cover any nv up to the
+ * limit of 2^31-2 vertices, and larger nv is rejected with
+ * NIDO_E_TOO_LARGE.  All calls on a device share the arrays: calls that
+ * overlap on the GPU race and return wrong values. */
 int nido_modularity_noalloc(void* stream, int64_t nv, const int64_t* d_off, const int64_t* d_adj,
                             const double* d_w, const int64_t* d_comm, const double* d_a, double m,
                             double* d_q);

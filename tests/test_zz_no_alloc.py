@@ -84,3 +84,46 @@ def test_noalloc_graph_without_edges(nido_lib, ctx):
     assert lib.nido_modularity_noalloc(None, nv, p(off), p(adj), p(w), p(comm), p(a), 1.0, p(q)) == 0
     torch.cuda.synchronize()
     assert float(q.item()) == 0.0
+
+
+def _star_graph(capi, nv, hub, leaves, seed):
+    """A vertex with `leaves` neighbours (edges split over several items) beside
+    a sparse ring, integer weights."""
+    rng = np.random.default_rng(seed)
+    u = np.concatenate([np.arange(nv - 1), np.full(leaves, hub)])
+    v = np.concatenate([np.arange(1, nv), rng.integers(0, nv, leaves)])
+    w = rng.integers(1, 9, len(u)).astype(np.float64)
+    keep = u != v
+    u, v, w = u[keep], v[keep], w[keep]
+    src, dst, ww = np.concatenate([u, v]), np.concatenate([v, u]), np.concatenate([w, w])
+    order = np.argsort(src, kind="stable")
+    off = np.zeros(nv + 1, np.int64)
+    np.cumsum(np.bincount(src, minlength=nv), out=off[1:])
+    return capi.Csr(off, dst[order].astype(np.int64), ww[order])
+
+
+# vertex counts at the edges of 16-vertex groups, 64-vertex tiles and the
+# search fan-out, hubs of none, one and several 4096-edge items, and more
+# vertices than thread slots (a second pass)
+@pytest.mark.parametrize("nv,hub,leaves", [(2, 0, 0), (17, 16, 3), (63, 5, 4095), (64, 63, 4096), (65, 64, 4097),
+                                           (257, 200, 20000), (16385, 16384, 50000), (65535 * 128 + 77, 1000, 30000)])
+def test_noalloc_tiles_match_oracle(nido_lib, ctx, orc, nv, hub, leaves):
+    import torch
+
+    capi = nido_lib
+    G = _star_graph(capi, nv, hub, leaves, 11)
+    comm = np.random.default_rng(12).integers(0, max(1, nv // 7), nv).astype(np.int64)
+    k = np.zeros(nv)
+    np.add.at(k, np.repeat(np.arange(nv), np.diff(G.off)), G.w)
+    a = np.zeros(nv)
+    np.add.at(a, comm, k)
+    m = float(k.sum() / 2)
+    d = [torch.from_numpy(x).to("cuda:0") for x in (G.off, G.adj, G.w, comm, a)]
+    d_q = torch.zeros(1, dtype=torch.float64, device="cuda:0")
+    torch.cuda.synchronize()
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    assert capi.lib().nido_modularity_noalloc(None, nv, *[p(t) for t in d], m, p(d_q)) == 0
+    torch.cuda.synchronize()
+    q, want = float(d_q.item()), orc.modularity(G.off, G.adj, G.w, comm, a, m)
+    # every sum is an integer, so any order is exact
+    assert np.float64(q).view(np.uint64) == np.float64(want).view(np.uint64), (q, want)
