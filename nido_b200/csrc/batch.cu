@@ -57,6 +57,7 @@ struct nido_batch_s {
   double* Qold = nullptr;
   double* qnew = nullptr;
   double* mg = nullptr;
+  double2* zg = nullptr;       // reciprocals of mg
   // work lists (graph ids and value offsets) and reduction buffers
   int32_t* plist = nullptr;    // graphs of the phase
   int32_t* llist = nullptr;    // graphs in the tier lists
@@ -200,6 +201,15 @@ __global__ void k_reduce_warp(const int32_t* __restrict__ gl, const int64_t* __r
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(NIDO_FULL_MASK, mine, o);
     if (lane == 0) out[gl[i]] = scale * mine;
+  }
+}
+
+__global__ void k_mass_recip(const int32_t* __restrict__ gl, int n, const double* __restrict__ mg,
+                             double2* __restrict__ zg) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double2 z;
+    mass_reciprocal(mg[gl[i]], &z.x, &z.y);
+    zg[gl[i]] = z;
   }
 }
 
@@ -540,7 +550,7 @@ extern "C" int nido_batch_free(nido_batch B) {
     for (void* p : {(void*)B->gbase0, (void*)B->gbA, (void*)B->gbB, (void*)B->gcuts, (void*)B->gparts,
                     (void*)B->gedges, (void*)B->gactive, (void*)B->giter, (void*)B->grest, (void*)B->gagg,
                     (void*)B->gfin, (void*)B->loops_phase, (void*)B->loops_total, (void*)B->phases, (void*)B->Q,
-                    (void*)B->Qold, (void*)B->qnew, (void*)B->mg, (void*)B->plist, (void*)B->llist,
+                    (void*)B->Qold, (void*)B->qnew, (void*)B->mg, (void*)B->zg, (void*)B->plist, (void*)B->llist,
                     (void*)B->moff, (void*)B->qoff, (void*)B->part, (void*)B->modv, (void*)B->selfv,
                     (void*)B->counters, (void*)B->bctl, (void*)B->gid, (void*)B->outc,
                     (void*)B->elist})
@@ -586,7 +596,7 @@ extern "C" int nido_batch_upload(nido_ctx ctx, int32_t ngraphs, const int64_t* v
   take(&B->gcuts, G * (nbatches + 1)); take(&B->gparts, G * (nbatches + 2)); take(&B->gedges, G);
   take(&B->gactive, G); take(&B->giter, G); take(&B->grest, G); take(&B->gagg, G); take(&B->gfin, G);
   take(&B->loops_phase, G); take(&B->loops_total, G); take(&B->phases, G);
-  take(&B->Q, G); take(&B->Qold, G); take(&B->qnew, G); take(&B->mg, G);
+  take(&B->Q, G); take(&B->Qold, G); take(&B->qnew, G); take(&B->mg, G); take(&B->zg, G);
   take(&B->plist, G); take(&B->llist, G); take(&B->moff, G + 1); take(&B->qoff, G + 1);
   take(&B->part, B->cap_part); take(&B->modv, B->cap_modv); take(&B->selfv, V);
   take(&B->counters, 4); take(&B->bctl, 16); take(&B->gid, V);
@@ -614,6 +624,7 @@ extern "C" int nido_batch_upload(nido_ctx ctx, int32_t ngraphs, const int64_t* v
   }
   g->gid = B->gid;
   g->mg = B->mg;
+  g->zg = B->zg;
   g->gcuts = B->gcuts;
   g->gactive = B->gactive;
   g->gbase = B->gbA;
@@ -718,6 +729,8 @@ extern "C" int nido_batch_run(nido_batch B, const nido_params* p, int64_t* out_c
                                                                                     g->gbase, g->k, B->part);
     NIDO_LAUNCH_CHECK();
     NIDO_TRY(reduce_lists(s, ml, B->plist, B->moff, B->part, 0.5, B->mg));
+    k_mass_recip<<<grid_for(np, 128), 128, 0, s>>>(B->plist, np, B->mg, B->zg);
+    NIDO_LAUNCH_CHECK();
     k_cuts_multi<<<grid_for(np, 128), 128, 0, s>>>(B->plist, np, g->off, g->gbase, nb, B->gcuts, B->gparts);
     NIDO_LAUNCH_CHECK();
     k_graph_edges<<<grid_for(ng, kThreads), kThreads, 0, s>>>(g->off, g->gbase, ng, B->gedges);

@@ -2,6 +2,7 @@
 #ifndef NIDO_COMMON_CUH_
 #define NIDO_COMMON_CUH_
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include "nido_b200.h"
@@ -59,6 +60,19 @@ __device__ __forceinline__ unsigned hash_slot(int c, unsigned mask) {
 // tree (graph_cuda.cu:1515-1526) prefers lanes on equal gains.
 __device__ __forceinline__ unsigned bitrev3(unsigned x) {
   return ((x & 1u) << 2) | (x & 2u) | ((x & 4u) >> 2);
+}
+
+// Reciprocal of a mass for quotients by it: zh = RN(1/m) and zl = (1 - m zh) zh,
+// or zeros when m lies outside 2^-400..2^400 (zero, infinities and NaN among
+// them) and the divide has to be used.
+__host__ __device__ inline void mass_reciprocal(double m, double* zh, double* zl) {
+  const double x = m < 0. ? -m : m;
+  *zh = 0.;
+  *zl = 0.;
+  if (!(x >= 0x1p-400 && x <= 0x1p400)) return;
+  const double r = 1.0 / m;
+  *zh = r;
+  *zl = fma(-m, r, 1.0) * r;
 }
 
 // "a beats b": larger gain, then smaller tie key (community id for the

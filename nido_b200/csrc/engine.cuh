@@ -199,6 +199,7 @@ struct nido_graph_s {
   // vertex's batch relative to its own graph's -b cuts
   int32_t* gid = nullptr;
   double* mg = nullptr;
+  double2* zg = nullptr;      // reciprocal of every graph's mass (mass_reciprocal)
   int32_t* vbatch = nullptr;
   int64_t* gbase = nullptr;   // first vertex of every graph (ngraphs+1)
   int64_t* gcuts = nullptr;   // -b cuts of every graph, relative (ngraphs*(nbatches+1))

@@ -48,6 +48,10 @@ struct MoveArgs {
   // one graph, whose mass is m)
   const int32_t* __restrict__ gid;
   const double* __restrict__ mg;
+  // integer phases: reciprocals of the mass (one graph) or of every graph's
+  // mass, RN(1/m) and its error term; {0, 0} where quotients by m need the divide
+  double zh, zl;
+  const double2* __restrict__ zg;
   // every weight integral and every vertex's sum of |w| below 2^31: the
   // shared-memory tables then add int32 (a native shared-memory atomic; the
   // FP64 one is several times slower) and every partial sum is exact, so
@@ -56,23 +60,52 @@ struct MoveArgs {
   int64_t nv;  // vertices of the current graph (all graphs in many-graph mode)
 };
 
+// The mass a vertex's gains are divided by, with its reciprocal zh = RN(1/m)
+// and zl = (1 - m zh) zh (zh = 0: use the divide).
+struct Mass {
+  double m, zh, zl;
+};
+
 // The mass of v's graph (kernels are instantiated per mode, so the
 // one-graph kernels carry no graph-id lookup).
 template <bool kMulti>
-__device__ __forceinline__ double vertex_mass(const MoveArgs& p, int v) {
-  return kMulti ? p.mg[p.gid[v]] : p.m;
+__device__ __forceinline__ Mass vertex_mass(const MoveArgs& p, int v) {
+  if constexpr (kMulti) {
+    const int g = p.gid[v];
+    const double2 z = p.zg ? p.zg[g] : make_double2(0., 0.);
+    return Mass{p.mg[g], z.x, z.y};
+  } else {
+    return Mass{p.m, p.zh, p.zl};
+  }
 }
 
 constexpr unsigned long long kNoKey = ~0ull;
 
-__device__ __forceinline__ double gain_of(double e, double ki, double ac, double m) {
-  const double t = __ddiv_rn(__dmul_rn(ki, ac), __dmul_rn(2.0, m));
-  return __ddiv_rn(__dsub_rn(e, t), m);
+// RN(a / m) from the reciprocal: q0 = RN(a zh + RN(a zl)) is within one ulp
+// of the quotient, its remainder a - m q0 is exact in one fused
+// multiply-add, and RN(q0 + remainder * zh) is the correctly rounded quotient
+// (P. W. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990, theorem 8.5).  Four multiply-adds instead of
+// a divide; every entry of every vertex needs two.  Only in integer phases:
+// their operands are 0 or between 2^-120 and 2^100, so nothing under- or
+// overflows; in FP64 phases the range checks cost what the divides do (sweeps
+// of a 250,007-vertex lognormal SBM: 1.634 ms with divides, 1.655 ms).
+__device__ __forceinline__ double div_mass(double a, const Mass& M) {
+  const double q0 = __fma_rn(a, M.zh, __dmul_rn(a, M.zl));
+  return __fma_rn(__fma_rn(-M.m, q0, a), M.zh, q0);
 }
 
-__device__ __forceinline__ double self_of(double eown, double ki, double aown, double m) {
-  const double t = __ddiv_rn(__dmul_rn(ki, __dsub_rn(aown, ki)), __dmul_rn(2.0, m));
-  return __ddiv_rn(__dsub_rn(eown, t), m);
+// (e - ki*ac/(2m)) / m in the reference's operation order; RN(y/(2m)) is
+// RN(y/m)/2 (a power of two).
+__device__ __forceinline__ double gain_of(double e, double ki, double ac, const Mass& M) {
+  const double y = __dmul_rn(ki, ac);
+  if (M.zh != 0.) return div_mass(__dsub_rn(e, __dmul_rn(0.5, div_mass(y, M))), M);
+  const double t = __ddiv_rn(y, __dmul_rn(2.0, M.m));
+  return __ddiv_rn(__dsub_rn(e, t), M.m);
+}
+
+__device__ __forceinline__ double self_of(double eown, double ki, double aown, const Mass& M) {
+  return gain_of(eown, ki, __dsub_rn(aown, ki), M);
 }
 
 __device__ __forceinline__ unsigned long long nido_key(unsigned rank) {
@@ -160,7 +193,8 @@ __global__ void __launch_bounds__(256, 6) k_move_group(const int32_t* __restrict
     const bool vok = idx < n;
     int v = 0, own = -1;
     int64_t s = 0, d = 0;
-    double ki = 0., aown = 0., m = p.m;
+    double ki = 0., aown = 0.;
+    Mass m{p.m, p.zh, p.zl};
     if (vok) {
       v = list[idx];
       s = p.off[v];
@@ -565,7 +599,7 @@ __device__ __forceinline__ void merge_edges_packed(const MoveArgs& p, int v, int
 // occ is null): e_own and the best (gain, tie key, community) of this thread.
 // Entries are taken four at a time so that their a_c gathers are in flight
 // together.
-__device__ __forceinline__ void scan_entries(const MoveArgs& p, double m, const Table& t, int n, int t0, int step,
+__device__ __forceinline__ void scan_entries(const MoveArgs& p, const Mass& m, const Table& t, int n, int t0, int step,
                                              int own, double ki, bool cg, double& eown, double& g,
                                              unsigned long long& tk, int& cand) {
   constexpr int U = 4;
@@ -607,7 +641,7 @@ __device__ __forceinline__ void scan_entries(const MoveArgs& p, double m, const 
 // The reference's tie rule over the same entries: among communities whose
 // gain equals gm, the smallest (bitrev3(rank mod 8), rank), where rank counts
 // the vertex's neighbour communities with a smaller id.
-__device__ __forceinline__ void nido_tie_entries(const MoveArgs& p, double m, const Table& t, int n, int t0, int step,
+__device__ __forceinline__ void nido_tie_entries(const MoveArgs& p, const Mass& m, const Table& t, int n, int t0, int step,
                                                  int own, double ki, double gm, bool cg, double& g,
                                                  unsigned long long& tk, int& cand) {
   g = -NIDO_MAX_FLOAT; tk = kNoKey; cand = -1;
@@ -628,7 +662,7 @@ __device__ __forceinline__ void nido_tie_entries(const MoveArgs& p, double m, co
   }
 }
 
-__device__ __forceinline__ void decide(const MoveArgs& p, double m, int v, int own, double ki, double aown, double eown,
+__device__ __forceinline__ void decide(const MoveArgs& p, const Mass& m, int v, int own, double ki, double aown, double eown,
                                        double g, int cand) {
   const double self = self_of(eown, ki, aown, m);
   const double tot = __dsub_rn(g, self);
@@ -677,7 +711,7 @@ __global__ void __launch_bounds__(256, 5) k_move_warp(const int32_t* __restrict_
     double g = -NIDO_MAX_FLOAT, eown = 0.;
     unsigned long long tk = kNoKey;
     int cand = -1;
-    const double m = vertex_mass<kMulti>(p, v);
+    const Mass m = vertex_mass<kMulti>(p, v);
     scan_entries(p, m, t, nu, lane, 32, own, ki, false, eown, g, tk, cand);
     eown = group_sum<32>(eown);
     if (p.tie == NIDO_TIE_NIDO) {
@@ -745,7 +779,7 @@ __device__ double block_max(double x, double* sx) {
 }
 
 // Evaluate a filled table with the whole block and write newc[v].
-__device__ __forceinline__ void block_evaluate(const MoveArgs& p, double m, const Table& t, int n, bool cg, int v, int own,
+__device__ __forceinline__ void block_evaluate(const MoveArgs& p, const Mass& m, const Table& t, int n, bool cg, int v, int own,
                                                double ki, double aown, double* sg, unsigned long long* stk,
                                                int* sc) {
   double g = -NIDO_MAX_FLOAT, eown = 0.;
@@ -1115,7 +1149,7 @@ __global__ void __launch_bounds__(kHubThreads) k_hub_slices(const int2* __restri
     double* vals = gvals + hub_toff[sl.x] + (int64_t)sl.y * kHubSlice;
     const int own = p.comm[v];
     const double ki = p.k[v];
-    const double m = vertex_mass<kMulti>(p, v);
+    const Mass m = vertex_mass<kMulti>(p, v);
     double g = -NIDO_MAX_FLOAT, eown = 0.;
     unsigned long long tk = kNoKey;
     int cand = -1;
@@ -1190,7 +1224,7 @@ __global__ void __launch_bounds__(kHubThreads) k_hub_slices_packed(const int2* _
     unsigned long long* slots = gslots + hub_toff[sl.x] + (int64_t)sl.y * kHubSlice;
     const int own = p.comm[v];
     const double ki = p.k[v];
-    const double m = vertex_mass<kMulti>(p, v);
+    const Mass m = vertex_mass<kMulti>(p, v);
     double g = -NIDO_MAX_FLOAT, eown = 0.;
     unsigned long long tk = kNoKey;
     int cand = -1;
@@ -1363,7 +1397,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_move_cluster(const int32_t* _
     }
     cluster.sync();  // every insert of this hub is in place
     const int own = p.comm[v];
-    const double ki = p.k[v], aown = p.a[own], m = vertex_mass<kMulti>(p, v);
+    const double ki = p.k[v], aown = p.a[own];
+    const Mass m = vertex_mass<kMulti>(p, v);
     double g = -NIDO_MAX_FLOAT, eown = 0.;
     unsigned long long tk = kNoKey;
     int cand = -1;
@@ -1876,8 +1911,12 @@ int move_init_attributes() {
 
 namespace {
 MoveArgs move_args(nido_graph_s* g, int tie) {
+  double zh = 0., zl = 0.;
+  if (!g->gid && g->int_weights) mass_reciprocal(g->m, &zh, &zl);
   return MoveArgs{g->off, g->adj, g->w, g->comm, g->k, g->a, g->newc, g->m, tie,
-                  reinterpret_cast<unsigned long long*>(g->dcount + 1), g->gid, g->mg, g->int_weights ? 1 : 0, g->nv};
+                  reinterpret_cast<unsigned long long*>(g->dcount + 1), g->gid, g->mg, zh, zl,
+                  g->int_weights ? g->zg : nullptr,
+                  g->int_weights ? 1 : 0, g->nv};
 }
 
 int tiers_direct(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
