@@ -27,460 +27,31 @@
 
 #include "common.cuh"
 #include "engine.cuh"
+#include "move_core.cuh"
+#include "move_tiers.cuh"
 
 namespace nido {
 namespace {
 
 namespace cg = cooperative_groups;
 
-struct MoveArgs {
-  const int64_t* __restrict__ off;
-  const int32_t* __restrict__ adj;
-  const double* __restrict__ w;
-  const int32_t* __restrict__ comm;
-  const double* __restrict__ k;
-  const double* __restrict__ a;
-  int32_t* __restrict__ newc;
-  double m;
-  int tie;
-  unsigned long long* err;  // probe-limit failures (never expected)
-  // many-graph mode: graph of every vertex and mass of every graph (null for
-  // one graph, whose mass is m)
-  const int32_t* __restrict__ gid;
-  const double* __restrict__ mg;
-  // integer phases: reciprocals of the mass (one graph) or of every graph's
-  // mass, RN(1/m) and its error term; {0, 0} where quotients by m need the divide
-  double zh, zl;
-  const double2* __restrict__ zg;
-  // every weight integral and every vertex's sum of |w| below 2^31: the
-  // shared-memory tables then add int32 (a native shared-memory atomic; the
-  // FP64 one is several times slower) and every partial sum is exact, so
-  // the e_vc read back are the FP64 sums bit for bit
-  int ints;
-  int64_t nv;  // vertices of the current graph (all graphs in many-graph mode)
-};
-
-// The mass a vertex's gains are divided by, with its reciprocal zh = RN(1/m)
-// and zl = (1 - m zh) zh (zh = 0: use the divide).
-struct Mass {
-  double m, zh, zl;
-};
-
-// The mass of v's graph (kernels are instantiated per mode, so the
-// one-graph kernels carry no graph-id lookup).
-template <bool kMulti>
-__device__ __forceinline__ Mass vertex_mass(const MoveArgs& p, int v) {
-  if constexpr (kMulti) {
-    const int g = p.gid[v];
-    const double2 z = p.zg ? p.zg[g] : make_double2(0., 0.);
-    return Mass{p.mg[g], z.x, z.y};
-  } else {
-    return Mass{p.m, p.zh, p.zl};
-  }
+// Self-check of the bounded waits: one thread waits on an mbarrier that
+// expects an arrival nobody makes.  The wait must give up and the kernel
+// report it (out[0] = 1, out[1] = milliseconds waited), leaving the context
+// usable.
+__global__ void k_check_bounded_wait(int32_t* out) {
+  __shared__ unsigned long long bar;
+  if (threadIdx.x != 0) return;
+  mbar_init(&bar, 1);
+  const unsigned long long t0 = gtimer_ns();
+  const bool done = mbar_wait(&bar, 0);
+  out[0] = done ? 0 : 1;
+  out[1] = (int32_t)min((gtimer_ns() - t0) / 1000000ull, 1ull << 30);
 }
 
-constexpr unsigned long long kNoKey = ~0ull;
-
-// RN(a / m) from the reciprocal: q0 = RN(a zh + RN(a zl)) is within one ulp
-// of the quotient, its remainder a - m q0 is exact in one fused
-// multiply-add, and RN(q0 + remainder * zh) is the correctly rounded quotient
-// (P. W. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990, theorem 8.5).  Four multiply-adds instead of
-// a divide; every entry of every vertex needs two.  Only in integer phases:
-// their operands are 0 or between 2^-120 and 2^100, so nothing under- or
-// overflows; in FP64 phases the range checks cost what the divides do (sweeps
-// of a 250,007-vertex lognormal SBM: 1.634 ms with divides, 1.655 ms).
-__device__ __forceinline__ double div_mass(double a, const Mass& M) {
-  const double q0 = __fma_rn(a, M.zh, __dmul_rn(a, M.zl));
-  return __fma_rn(__fma_rn(-M.m, q0, a), M.zh, q0);
-}
-
-// (e - ki*ac/(2m)) / m in the reference's operation order; RN(y/(2m)) is
-// RN(y/m)/2 (a power of two).
-__device__ __forceinline__ double gain_of(double e, double ki, double ac, const Mass& M) {
-  const double y = __dmul_rn(ki, ac);
-  if (M.zh != 0.) return div_mass(__dsub_rn(e, __dmul_rn(0.5, div_mass(y, M))), M);
-  const double t = __ddiv_rn(y, __dmul_rn(2.0, M.m));
-  return __ddiv_rn(__dsub_rn(e, t), M.m);
-}
-
-__device__ __forceinline__ double self_of(double eown, double ki, double aown, const Mass& M) {
-  return gain_of(eown, ki, __dsub_rn(aown, ki), M);
-}
-
-__device__ __forceinline__ unsigned long long nido_key(unsigned rank) {
-  return ((unsigned long long)bitrev3(rank & 7u) << 32) | rank;
-}
-
-// Sum of `wt` over the lanes in `peers`, in ascending lane order (a left fold
-// in edge order).  Every lane of the warp must call it.
-__device__ __forceinline__ double fold_peers(unsigned peers, bool ok, double wt) {
-  const int lane = threadIdx.x & 31;
-  unsigned rem = ok ? peers : 0u;
-  const int maxcnt = __reduce_max_sync(NIDO_FULL_MASK, (unsigned)__popc(rem));
-  double e = 0.;
-  for (int i = 0; i < maxcnt; ++i) {
-    const int src = rem ? __ffs(rem) - 1 : lane;
-    const double x = __shfl_sync(NIDO_FULL_MASK, wt, src);
-    if (rem) {
-      e += x;
-      rem &= rem - 1;
-    }
-  }
-  return e;
-}
-
-// Butterfly argmax over groups of G lanes (every lane ends with the result).
-template <int G>
-__device__ __forceinline__ void group_best(double& g, unsigned long long& tk, int& cand) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) {
-    const double g2 = __shfl_xor_sync(NIDO_FULL_MASK, g, o, G);
-    const unsigned long long t2 = __shfl_xor_sync(NIDO_FULL_MASK, tk, o, G);
-    const int c2 = __shfl_xor_sync(NIDO_FULL_MASK, cand, o, G);
-    if (better(g2, t2, g, tk)) { g = g2; tk = t2; cand = c2; }
-  }
-}
-
-template <int G>
-__device__ __forceinline__ double group_max(double g) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) g = fmax(g, __shfl_xor_sync(NIDO_FULL_MASK, g, o, G));
-  return g;
-}
-
-template <int G>
-__device__ __forceinline__ double group_sum(double x) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) x += __shfl_xor_sync(NIDO_FULL_MASK, x, o, G);
-  return x;
-}
-
-// Warp argmax of (gain, smallest id) under the smallest-id rule (tk is the
-// community id, kNoKey without a candidate) with three 32-bit warp
-// reductions instead of a shuffle tree: the gain as an order-preserving
-// 64-bit key (+0 for -0, which compares equal to it), then the smallest id
-// among the lanes holding the largest gain.  The result is group_best<32>'s.
-// Every lane of the warp must call it; all end with the result.
-__device__ __forceinline__ void warp_best_id(double& g, unsigned long long& tk, int& cand) {
-  const long long b = __double_as_longlong(g + 0.0);
-  const unsigned long long key = b < 0 ? ~(unsigned long long)b : ((unsigned long long)b | 0x8000000000000000ull);
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned mh = __reduce_max_sync(NIDO_FULL_MASK, hi);
-  const unsigned ml = __reduce_max_sync(NIDO_FULL_MASK, hi == mh ? lo : 0u);
-  const bool top = hi == mh && lo == ml;
-  const unsigned id = tk == kNoKey ? 0xFFFFFFFFu : (unsigned)tk;
-  const unsigned mid = __reduce_min_sync(NIDO_FULL_MASK, top ? id : 0xFFFFFFFFu);
-  const int src = __ffs(__ballot_sync(NIDO_FULL_MASK, top && id == mid)) - 1;
-  g = __shfl_sync(NIDO_FULL_MASK, g, src);
-  tk = __shfl_sync(NIDO_FULL_MASK, tk, src);
-  cand = __shfl_sync(NIDO_FULL_MASK, cand, src);
-}
-
-// ---- degree <= 32: registers ---------------------------------------------------
-// Six 256-thread blocks an SM (at most 40 registers a thread): the tier waits
-// on its gathers, and more resident warps hide more of them.
-template <int G, bool kMulti>
-__global__ void __launch_bounds__(256, 6) k_move_group(const int32_t* __restrict__ list, int64_t n,
-                                                    MoveArgs p) {
-  constexpr int VPW = 32 / G;
-  __shared__ int fold[256];  // integer phases: per-lane group sums
-  const int lane = threadIdx.x & 31, gl = lane & (G - 1), gid = lane / G;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t b = warp * VPW; b < n; b += nw * VPW) {
-    const int64_t idx = b + gid;
-    const bool vok = idx < n;
-    int v = 0, own = -1;
-    int64_t s = 0, d = 0;
-    double ki = 0., aown = 0.;
-    Mass m{p.m, p.zh, p.zl};
-    if (vok) {
-      v = list[idx];
-      s = p.off[v];
-      d = p.off[v + 1] - s;
-      own = p.comm[v];
-      ki = p.k[v];
-      aown = p.a[own];
-      m = vertex_mass<kMulti>(p, v);
-    }
-    const bool ok = gl < d;
-    int c = -1;
-    double wt = 0.;
-    if (ok) {
-      const int u = p.adj[s + gl];
-      c = p.comm[u];
-      wt = (u == v) ? 0. : p.w[s + gl];
-    }
-    // lanes of one vertex with equal communities: a 32-bit match where the
-    // group index fits above the ids (invalid lanes, c = -1, may match across
-    // groups; they add nothing), else a 64-bit one
-    unsigned peers;
-    if constexpr (G == 32) {
-      peers = __match_any_sync(NIDO_FULL_MASK, (unsigned)c);
-    } else if (p.nv <= (int64_t)1 << 29) {
-      peers = __match_any_sync(NIDO_FULL_MASK, (unsigned)c | ((unsigned)gid << 29));
-    } else {
-      peers = __match_any_sync(NIDO_FULL_MASK, ((unsigned long long)(unsigned)gid << 32) | (unsigned)c);
-    }
-    const int leader = __ffs(peers) - 1;
-    const bool lead = ok && lane == leader;
-    double e;
-    if (p.ints) {
-      // integer weights: every lane adds its weight into its group leader's
-      // shared-memory slot (int32 adds, exact in any order; equal addresses
-      // are serialised by the atomic unit, not by instructions)
-      fold[threadIdx.x] = 0;
-      __syncwarp();
-      if (ok) atomicAdd(&fold[(threadIdx.x & ~31) + leader], __double2int_rn(wt));
-      __syncwarp();
-      e = (double)fold[threadIdx.x];
-    } else {
-      e = fold_peers(peers, ok, wt);
-    }
-    double g = -NIDO_MAX_FLOAT, eown = 0.;
-    unsigned long long tk = kNoKey;
-    int cand = -1;
-    if (lead) {
-      if (c == own) {
-        eown = e;
-      } else {
-        g = gain_of(e, ki, p.a[c], m);
-        tk = (unsigned)c;
-        cand = c;
-      }
-    }
-    eown = group_sum<G>(eown);
-    if (p.tie == NIDO_TIE_NIDO) {
-      const double gm = group_max<G>(g);
-      unsigned rank = 0;
-      const int gbase = gid * G;
-      for (int j = 0; j < G; ++j) {
-        const int cj = __shfl_sync(NIDO_FULL_MASK, c, gbase + j);
-        const int lj = __shfl_sync(NIDO_FULL_MASK, (int)lead, gbase + j);
-        rank += (lj && cj < c) ? 1u : 0u;
-      }
-      tk = (cand >= 0 && g == gm) ? nido_key(rank) : kNoKey;
-      if (tk == kNoKey) { g = -NIDO_MAX_FLOAT; cand = -1; }
-    }
-    if (G == 32 && p.tie != NIDO_TIE_NIDO) warp_best_id(g, tk, cand);
-    else group_best<G>(g, tk, cand);
-    if (gl == 0 && vok) {
-      const double self = self_of(eown, ki, aown, m);
-      const double tot = __dsub_rn(g, self);
-      p.newc[v] = (cand >= 0 && tot > 0.) ? cand : own;
-    }
-  }
-}
-
-
-// ---- hash tables --------------------------------------------------------------
-// Open addressing over a power-of-two slot array.  New keys are appended to an
-// occupied-slot list so that evaluation and clearing cost O(unique keys).
-// Tables hold at least twice as many slots as the vertex has edges, so a free
-// slot always exists; probing is still bounded by the table size, and a full
-// table is reported through *err.
-struct Table {
-  int* keys;
-  double* vals;  // FP64 values, or with ints the int32 sum in each slot's low word
-  int* occ;
-  int* nocc;
-  unsigned mask;
-  bool ints = false;  // shared-memory tables of integer-weight phases
-  // integer-weight phases in shared memory: one 64-bit word a slot, the
-  // community id in the high half (-1: empty) and the int32 sum in the low
-  // half, so an insert and its first add are one compare-and-swap (keys and
-  // vals are unused then)
-  unsigned long long* slots = nullptr;
-};
-
-constexpr unsigned long long kEmptySlot = 0xFFFFFFFF00000000ull;
-__device__ __forceinline__ int slot_key(unsigned long long x) { return (int)(x >> 32); }
-__device__ __forceinline__ int slot_sum(unsigned long long x) { return (int)(unsigned)x; }
-
-__device__ __forceinline__ int* int_slot(const Table& t, unsigned h) { return reinterpret_cast<int*>(t.vals + h); }
-
-// e_vc of a slot of a shared-memory table
-__device__ __forceinline__ double table_val(const Table& t, int slot) {
-  if (t.slots) return (double)slot_sum(t.slots[slot]);
-  return t.ints ? (double)*int_slot(t, (unsigned)slot) : t.vals[slot];
-}
-
-__device__ __forceinline__ int table_key(const Table& t, int slot) {
-  return t.slots ? slot_key(t.slots[slot]) : t.keys[slot];
-}
-
-// Adds the integer w to key c's sum in a packed table, inserting c when
-// absent (the insert carries w); returns the slot.  Sums are int32 adds on
-// the slot's low half, exact in any order (integer weights, every vertex's
-// sum of |w| below 2^31).
-__device__ __forceinline__ int table_add_packed(const Table& t, int c, int w, bool& isnew, unsigned long long* err) {
-  unsigned h = hash_slot(c, t.mask);
-  volatile unsigned long long* vs = t.slots;
-  isnew = false;
-  for (unsigned probe = 0; probe <= t.mask; ++probe) {
-    int k = slot_key(vs[h]);
-    if (k == -1) {
-      const unsigned long long mine = ((unsigned long long)(unsigned)c << 32) | (unsigned)w;
-      const unsigned long long old = atomicCAS(&t.slots[h], kEmptySlot, mine);
-      if (old == kEmptySlot) {
-        isnew = true;
-        return (int)h;
-      }
-      k = slot_key(old);
-    }
-    if (k == c) {
-      atomicAdd(reinterpret_cast<int*>(&t.slots[h]), w);
-      return (int)h;
-    }
-    h = (h + probe + 1) & t.mask;  // triangular steps: every slot once
-  }
-  atomicAdd(err, 1ull);
-  return -1;
-}
-
-// Adds e to key c's value, inserting c when absent; returns the slot and
-// whether this call inserted it.  Tables in global memory (kGlobal) go
-// straight to the compare-and-swap, one L2 round trip per probe; shared-memory
-// tables read the key first.
-template <bool kAtomicVals, bool kGlobal = false>
-__device__ __forceinline__ int table_add(const Table& t, int c, double e, bool& isnew, unsigned long long* err) {
-  unsigned h = hash_slot(c, t.mask);
-  volatile int* vk = t.keys;
-  isnew = false;
-  for (unsigned probe = 0; probe <= t.mask; ++probe) {
-    if constexpr (kGlobal) {
-      const int old = atomicCAS(&t.keys[h], -1, c);
-      if (old == -1 || old == c) {
-        isnew = old == -1;
-        atomicAdd(&t.vals[h], e);
-        return (int)h;
-      }
-      h = (h + 1) & t.mask;
-      continue;
-    }
-    const int kk = vk[h];
-    bool hit = kk == c;
-    if (!hit && kk == -1) {
-      const int old = atomicCAS(&t.keys[h], -1, c);
-      isnew = old == -1;
-      hit = isnew || old == c;
-    }
-    if (hit) {
-      if (t.ints) {
-        if (kAtomicVals) atomicAdd(int_slot(t, h), __double2int_rn(e));
-        else *int_slot(t, h) += __double2int_rn(e);
-      } else {
-        if (kAtomicVals) atomicAdd(&t.vals[h], e);
-        else t.vals[h] += e;
-      }
-      return (int)h;
-    }
-    h = (h + probe + 1) & t.mask;  // triangular steps: every slot once
-  }
-  atomicAdd(err, 1ull);
-  return -1;
-}
-
-// Appends the slots this warp inserted to the occupied list with one atomic
-// per warp.  Every lane of the warp must call it.
-__device__ __forceinline__ void occ_append(const Table& t, bool isnew, int slot) {
-  const unsigned nb = __ballot_sync(NIDO_FULL_MASK, isnew);
-  if (nb == 0u || t.occ == nullptr) return;
-  const int lane = threadIdx.x & 31, leader = __ffs(nb) - 1;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(t.nocc, __popc(nb));
-  base = __shfl_sync(NIDO_FULL_MASK, base, leader);
-  if (isnew) t.occ[base + __popc(nb & lanemask_lt())] = slot;
-}
-
-// Edge ids and weights are read once per sweep: loaded without allocating in
-// L1, which keeps L1 for the comm[u] and a[c] gathers (-2% on the move phase).
-__device__ __forceinline__ int ld_stream(const int* q) {
-  int v;
-  asm("ld.global.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(q));
-  return v;
-}
-__device__ __forceinline__ double ld_stream(const double* q) {
-  double v;
-  asm("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(q));
-  return v;
-}
-
-// smallest power of two >= max(64, 2d) (shared-memory tiers: d <= 2^30)
-__device__ __forceinline__ unsigned next_pow2_cap(int64_t d) {
-  const unsigned x = (unsigned)max((int64_t)64, 2 * min(d, (int64_t)1 << 30));
-  return 1u << (32 - __clz(x - 1));
-}
-
-// Accumulate the edges [first, eend) of vertex v: the warp takes 32-edge
-// chunks at first, first+stride, ...  kUnroll chunks are loaded (ids, weights,
-// then the communities) before any is merged, so each warp keeps several
-// dependent gathers in flight.  Chunks are merged in order.  Every lane of the
-// warp takes part.
-// The edges come from global memory, or (sadj non-null) from a copy of the
-// vertex's ranges in shared memory: edge j at sadj[j - a0] and sw[j - w0].
-template <bool kAtomicVals, int kUnroll, bool kGlobal = false>
-__device__ __forceinline__ void accumulate_edges(const MoveArgs& p, int v, int64_t first, int64_t eend,
-                                                 int64_t stride, const Table& t, const int32_t* sadj = nullptr,
-                                                 const double* sw = nullptr, int64_t a0 = 0, int64_t w0 = 0) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t base = first; base < eend; base += kUnroll * stride) {
-    int u[kUnroll], c[kUnroll];
-    double wt[kUnroll];
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      const int64_t j = base + k * stride + lane;
-      u[k] = -1;
-      wt[k] = 0.;
-      if (j < eend) {
-        if (sadj) {
-          u[k] = sadj[j - a0];
-          wt[k] = sw[j - w0];
-        } else {
-          u[k] = ld_stream(p.adj + j);
-          wt[k] = ld_stream(p.w + j);
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      c[k] = u[k] >= 0 ? p.comm[u[k]] : -1;
-      if (u[k] == v) wt[k] = 0.;
-    }
-    if (!kGlobal && t.slots) {
-      // packed integer table: every lane adds its own edge (native 32-bit
-      // shared-memory atomics, exact in any order), no fold across lanes
-#pragma unroll
-      for (int k = 0; k < kUnroll; ++k) {
-        const bool ok = u[k] >= 0;
-        if (!__any_sync(NIDO_FULL_MASK, ok)) break;
-        bool isnew = false;
-        int slot = -1;
-        if (ok) slot = table_add_packed(t, c[k], __double2int_rn(wt[k]), isnew, p.err);
-        occ_append(t, isnew, slot);
-        __syncwarp();
-      }
-      continue;
-    }
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      const bool ok = u[k] >= 0;
-      if (!__any_sync(NIDO_FULL_MASK, ok)) break;
-      const unsigned peers = __match_any_sync(NIDO_FULL_MASK, c[k]);
-      const bool lead = ok && lane == __ffs(peers) - 1;
-      const double e = fold_peers(peers, ok, wt[k]);
-      bool isnew = false;
-      int slot = -1;
-      if (lead) slot = table_add<kAtomicVals, kGlobal>(t, c[k], e, isnew, p.err);
-      occ_append(t, isnew, slot);
-      if (!kAtomicVals) __syncwarp();
-    }
-  }
-}
-
-// Hub segments (smallest-id rule): like accumulate_edges into a global
-// table, but every lane keeps the compare-and-swaps of its kUnroll chunks in
+// ---- hub tables in global memory ------------------------------------------------
+// Hub segments: the edges [first, eend) of vertex v in 32-edge chunks into a
+// global table; every lane keeps the compare-and-swaps of its kUnroll chunks in
 // flight together instead of finishing one chunk's probe before the next.
 // Equal communities within a chunk are still folded onto one lane first.
 template <int kUnroll>
@@ -595,148 +166,6 @@ __device__ __forceinline__ void merge_edges_packed(const MoveArgs& p, int v, int
   }
 }
 
-// Scan entries i = t0, t0+step, ... of the occupied list (or of all slots when
-// occ is null): e_own and the best (gain, tie key, community) of this thread.
-// Entries are taken four at a time so that their a_c gathers are in flight
-// together.
-__device__ __forceinline__ void scan_entries(const MoveArgs& p, const Mass& m, const Table& t, int n, int t0, int step,
-                                             int own, double ki, bool cg, double& eown, double& g,
-                                             unsigned long long& tk, int& cand) {
-  constexpr int U = 4;
-  for (int i = t0; i < n; i += U * step) {
-    int cc[U];
-    double val[U], ac[U];
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const int ii = i + k * step;
-      cc[k] = -1;
-      if (ii < n) {
-        const int slot = t.occ ? t.occ[ii] : ii;
-        if (t.slots) {
-          const unsigned long long x = t.slots[slot];
-          cc[k] = slot_key(x);
-          val[k] = (double)slot_sum(x);
-        } else {
-          cc[k] = cg ? __ldcg(&t.keys[slot]) : t.keys[slot];
-          val[k] = cg ? __ldcg(&t.vals[slot]) : table_val(t, slot);
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < U; ++k) ac[k] = (cc[k] >= 0 && cc[k] != own) ? p.a[cc[k]] : 0.;
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      if (cc[k] < 0) continue;
-      if (cc[k] == own) {
-        eown = val[k];
-      } else {
-        const double gg = gain_of(val[k], ki, ac[k], m);
-        if (better(gg, (unsigned)cc[k], g, tk)) { g = gg; tk = (unsigned)cc[k]; cand = cc[k]; }
-      }
-    }
-  }
-}
-
-
-// The reference's tie rule over the same entries: among communities whose
-// gain equals gm, the smallest (bitrev3(rank mod 8), rank), where rank counts
-// the vertex's neighbour communities with a smaller id.
-__device__ __forceinline__ void nido_tie_entries(const MoveArgs& p, const Mass& m, const Table& t, int n, int t0, int step,
-                                                 int own, double ki, double gm, bool cg, double& g,
-                                                 unsigned long long& tk, int& cand) {
-  g = -NIDO_MAX_FLOAT; tk = kNoKey; cand = -1;
-  for (int i = t0; i < n; i += step) {
-    const int slot = t.occ ? t.occ[i] : i;
-    const int cc = cg ? __ldcg(&t.keys[slot]) : table_key(t, slot);
-    if (cc < 0 || cc == own) continue;
-    const double val = cg ? __ldcg(&t.vals[slot]) : table_val(t, slot);
-    if (gain_of(val, ki, p.a[cc], m) != gm) continue;
-    unsigned rank = 0;
-    for (int q = 0; q < n; ++q) {
-      const int sq = t.occ ? t.occ[q] : q;
-      const int kq = cg ? __ldcg(&t.keys[sq]) : table_key(t, sq);
-      rank += (kq >= 0 && kq < cc) ? 1u : 0u;
-    }
-    const unsigned long long key = nido_key(rank);
-    if (key < tk) { tk = key; cand = cc; g = gm; }
-  }
-}
-
-__device__ __forceinline__ void decide(const MoveArgs& p, const Mass& m, int v, int own, double ki, double aown, double eown,
-                                       double g, int cand) {
-  const double self = self_of(eown, ki, aown, m);
-  const double tot = __dsub_rn(g, self);
-  p.newc[v] = (cand >= 0 && tot > 0.) ? cand : own;
-}
-
-// ---- 32 < degree <= 256: one warp per vertex, table in shared memory -----------
-// Shared memory of the tables: FP64 tables hold 8-byte values, 4-byte keys
-// and a 4-byte occupied list (16 bytes a slot); packed integer tables 8-byte
-// slots and the occupied list (12 bytes a slot).
-constexpr size_t table_bytes(int slots, bool ints) { return (size_t)slots * (ints ? 12 : 16); }
-
-// Five 256-thread blocks an SM (at most 48 registers a thread; a few spill).
-template <int kCap, bool kMulti, bool kInts>
-__global__ void __launch_bounds__(256, 5) k_move_warp(const int32_t* __restrict__ list, int64_t n, MoveArgs p) {
-  extern __shared__ double smem[];
-  __shared__ int nocc_s[8];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  Table t;
-  if constexpr (kInts) {
-    t.slots = reinterpret_cast<unsigned long long*>(smem) + (size_t)wid * kCap;
-    t.keys = nullptr;
-    t.vals = nullptr;
-    t.occ = reinterpret_cast<int*>(smem + 8 * kCap) + (size_t)wid * kCap;
-    for (int i = lane; i < kCap; i += 32) t.slots[i] = kEmptySlot;
-  } else {
-    t.vals = smem + (size_t)wid * kCap;
-    t.keys = reinterpret_cast<int*>(smem + 8 * kCap) + (size_t)wid * 2 * kCap;
-    t.occ = t.keys + kCap;
-    for (int i = lane; i < kCap; i += 32) { t.keys[i] = -1; t.vals[i] = 0.; }
-  }
-  t.nocc = &nocc_s[wid];
-  t.ints = kInts;
-  if (lane == 0) *t.nocc = 0;
-  __syncwarp();
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t task = warp; task < n; task += nw) {
-    const int v = list[task];
-    const int64_t s = p.off[v], eend = p.off[v + 1];
-    t.mask = min((unsigned)kCap, next_pow2_cap(eend - s)) - 1;
-    const int own = p.comm[v];
-    const double ki = p.k[v], aown = p.a[own];
-    accumulate_edges<false, 4>(p, v, s, eend, 32, t);
-    const int nu = *t.nocc;
-    double g = -NIDO_MAX_FLOAT, eown = 0.;
-    unsigned long long tk = kNoKey;
-    int cand = -1;
-    const Mass m = vertex_mass<kMulti>(p, v);
-    scan_entries(p, m, t, nu, lane, 32, own, ki, false, eown, g, tk, cand);
-    eown = group_sum<32>(eown);
-    if (p.tie == NIDO_TIE_NIDO) {
-      const double gm = group_max<32>(g);
-      nido_tie_entries(p, m, t, nu, lane, 32, own, ki, gm, false, g, tk, cand);
-      group_best<32>(g, tk, cand);
-    } else {
-      warp_best_id(g, tk, cand);
-    }
-    if (lane == 0) decide(p, m, v, own, ki, aown, eown, g, cand);
-    __syncwarp();
-    for (int i = lane; i < nu; i += 32) {
-      const int slot = t.occ[i];
-      if constexpr (kInts) {
-        t.slots[slot] = kEmptySlot;
-      } else {
-        t.keys[slot] = -1;
-        t.vals[slot] = 0.;
-      }
-    }
-    if (lane == 0) *t.nocc = 0;
-    __syncwarp();
-  }
-}
-
 // Block-wide argmax: every thread gets the result.
 __device__ void block_best(double& g, unsigned long long& tk, int& cand, double* sg,
                            unsigned long long* stk, int* sc) {
@@ -778,265 +207,83 @@ __device__ double block_max(double x, double* sx) {
   return t;
 }
 
-// Evaluate a filled table with the whole block and write newc[v].
-__device__ __forceinline__ void block_evaluate(const MoveArgs& p, const Mass& m, const Table& t, int n, bool cg, int v, int own,
-                                               double ki, double aown, double* sg, unsigned long long* stk,
-                                               int* sc) {
-  double g = -NIDO_MAX_FLOAT, eown = 0.;
-  unsigned long long tk = kNoKey;
-  int cand = -1;
-  scan_entries(p, m, t, n, threadIdx.x, blockDim.x, own, ki, cg, eown, g, tk, cand);
-  if (p.tie == NIDO_TIE_NIDO) {
-    eown = block_sum(eown, sg);
-    const double gm = block_max(g, sg);
-    nido_tie_entries(p, m, t, n, threadIdx.x, blockDim.x, own, ki, gm, cg, g, tk, cand);
-  }
-  // one reduction for the best entry and e_own (e_own is nonzero in one
-  // thread at most, so its sum is exact in any order)
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (p.tie != NIDO_TIE_NIDO) {
-    eown = group_sum<32>(eown);
-    warp_best_id(g, tk, cand);
-  } else {
-    group_best<32>(g, tk, cand);
-  }
-  __shared__ double se[32];
-  if (lane == 0) { sg[wid] = g; stk[wid] = tk; sc[wid] = cand; se[wid] = eown; }
-  __syncthreads();
-  if (wid == 0) {
-    g = lane < nw ? sg[lane] : -NIDO_MAX_FLOAT;
-    tk = lane < nw ? stk[lane] : kNoKey;
-    cand = lane < nw ? sc[lane] : -1;
-    double e2 = lane < nw ? se[lane] : 0.;
-    if (p.tie != NIDO_TIE_NIDO) warp_best_id(g, tk, cand);
-    else group_best<32>(g, tk, cand);
-    e2 = group_sum<32>(e2);
-    if (lane == 0) decide(p, m, v, own, ki, aown, p.tie == NIDO_TIE_NIDO ? eown : e2, g, cand);
-  }
-}
-
-// ---- staged adjacency: 1-D bulk copies (TMA) of a vertex's edge ranges --------
-// One thread copies the next vertex's ids and weights from this GPU's global
-// memory into shared memory with cp.async.bulk, completed on an mbarrier,
-// while the block still evaluates the current vertex; the block then reads
-// the edges from shared memory.  Copies start and end on 16-byte boundaries:
-// the id range is widened to multiples of 4 ids and the weight range to
-// multiples of 2 weights (the edge arrays carry 4 spare entries so the widened
-// end stays inside them).  No multicast.
-__device__ __forceinline__ unsigned smem_u32(const void* ptr) { return (unsigned)__cvta_generic_to_shared(ptr); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred P;\n mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n selp.u32 %0, 1, 0, P;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ unsigned long long gtimer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// bounded wait: gives up (false) after kMbarTries attempts or about a second,
-// whichever comes first, instead of spinning forever; the caller counts the
-// failure in p.err
-constexpr int kMbarTries = 1 << 20;
-constexpr unsigned long long kMbarWaitNs = 1000000000ull;
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
-  const unsigned long long t0 = gtimer_ns();
-  for (int i = 0; i < kMbarTries; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255) == 255 && gtimer_ns() - t0 > kMbarWaitNs) return false;
-  }
-  return false;
-}
-
-// Self-check of the bounded waits: one thread waits on an mbarrier that
-// expects an arrival nobody makes.  The wait must give up and the kernel
-// report it (out[0] = 1, out[1] = milliseconds waited), leaving the context
-// usable.
-__global__ void k_check_bounded_wait(int32_t* out) {
-  __shared__ unsigned long long bar;
-  if (threadIdx.x != 0) return;
-  mbar_init(&bar, 1);
-  const unsigned long long t0 = gtimer_ns();
-  const bool done = mbar_wait(&bar, 0);
-  out[0] = done ? 0 : 1;
-  out[1] = (int32_t)min((gtimer_ns() - t0) / 1000000ull, 1ull << 30);
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-// shared memory of one staged vertex of degree <= kDeg: ids then weights
-template <int kDeg>
-struct Stage {
-  static constexpr int kIds = kDeg + 8;     // widened by up to 3 ids each side
-  static constexpr int kWts = kDeg + 4;     // widened by up to 1 weight each side
-  static constexpr size_t kBytes = (size_t)kIds * 4 + (size_t)kWts * 8;
+// A hub's FP64 table (the reference's tie rule): cap = mask + 1 slots.
+struct Table {
+  int* keys;
+  double* vals;
+  unsigned mask;
 };
 
-// Thread 0: copy the edges [s, e) into the stage (ids at sadj, weights at
-// sw) on bar; *a0 / *w0 receive the first id / weight index held.
-__device__ __forceinline__ void stage_edges(const MoveArgs& p, int64_t s, int64_t e, int32_t* sadj, double* sw,
-                                            unsigned long long* bar, int64_t* a0, int64_t* w0) {
-  const int64_t ia = s & ~(int64_t)3, ib = (e + 3) & ~(int64_t)3;
-  const int64_t wa = s & ~(int64_t)1, wb = (e + 1) & ~(int64_t)1;
-  const unsigned bi = (unsigned)(4 * (ib - ia)), bw = (unsigned)(8 * (wb - wa));
-  *a0 = ia;
-  *w0 = wa;
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the stage come first
-  mbar_arrive_expect_tx(bar, bi + bw);
-  if (bi) bulk_g2s(sadj, p.adj + ia, bi, bar);
-  if (bw) bulk_g2s(sw, p.w + wa, bw, bar);
+// Scan the slots t0, t0+step, ... of a hub's table: e_own and the best (gain, id)
+// of this thread.  Slots are taken four at a time so that their a_c gathers are
+// in flight together.
+__device__ __forceinline__ void scan_slots(const MoveArgs& p, const Mass& m, const Table& t, int own, double ki,
+                                           double& eown, double& g, unsigned& id) {
+  constexpr int U = 4;
+  const int n = (int)t.mask + 1, step = (int)blockDim.x;
+  for (int i = threadIdx.x; i < n; i += U * step) {
+    int cc[U];
+    double val[U], ac[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int ii = i + k * step;
+      cc[k] = -1;
+      if (ii < n) {
+        cc[k] = __ldcg(&t.keys[ii]);
+        val[k] = __ldcg(&t.vals[ii]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) ac[k] = (cc[k] >= 0 && cc[k] != own) ? p.a[cc[k]] : 0.;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (cc[k] < 0) continue;
+      if (cc[k] == own) {
+        eown = val[k];
+      } else {
+        const double gg = gain_of(val[k], ki, ac[k], m);
+        if (gg > g || (gg == g && (unsigned)cc[k] < id)) { g = gg; id = (unsigned)cc[k]; }
+      }
+    }
+  }
 }
 
-// ---- 256 < degree <= 2048: one CTA per vertex, table in shared memory ----------
-// kOcc: keep a list of occupied slots (16 bytes a slot) so evaluation and
-// clearing touch only used slots; without it (12 bytes a slot, for the
-// largest FP64 table) both walk the vertex's whole table.  Packed integer
-// tables (kInts) always keep the list: 12 bytes a slot with it.
-// kStageDeg > 0: the tier's vertices (degree <= kStageDeg) have their edges
-// staged in shared memory behind the table (see stage_edges), one vertex
-// ahead: the copy of vertex i+1 runs while vertex i is evaluated.
-// Resident CTAs an SM: ten of 128 threads or five of 256 (at most 48 registers
-// a thread), else the 64-register fill of 1024 threads.
-template <int kThreads, int kCap, bool kMulti, bool kInts, bool kOcc = true, int kStageDeg = 0>
-__global__ void __launch_bounds__(kThreads, kThreads == 128 ? 10 : (kThreads == 256 ? 5 : 1024 / kThreads)) k_move_cta(const int32_t* __restrict__ list, int64_t n, MoveArgs p) {
-  constexpr bool kList = kOcc || kInts;
-  constexpr bool kStaged = kStageDeg > 0;
-  extern __shared__ __align__(128) double smem[];
-  __shared__ double sg[32];
-  __shared__ unsigned long long stk[32];
-  __shared__ int sc[32];
-  __shared__ int nocc_s;
-  __shared__ unsigned long long stage_bar;
-  __shared__ long long stage_off[2];  // first id and weight index held by the stage
-  int32_t* sadj = nullptr;
-  double* sw = nullptr;
-  if constexpr (kStaged) {
-    char* st = reinterpret_cast<char*>(smem) + table_bytes(kCap, kInts);
-    sadj = reinterpret_cast<int32_t*>(st);
-    sw = reinterpret_cast<double*>(st + (size_t)Stage<kStageDeg>::kIds * 4);
-    if (threadIdx.x == 0) {
-      mbar_init(&stage_bar, 1);
-      if (blockIdx.x < n) {  // the first vertex's edges start on their way at once
-        const int v0 = list[blockIdx.x];
-        int64_t a0, w0;
-        stage_edges(p, p.off[v0], p.off[v0 + 1], sadj, sw, &stage_bar, &a0, &w0);
-        stage_off[0] = a0;
-        stage_off[1] = w0;
-      }
+// The reference's tie rule over the same slots: among communities whose
+// gain equals gm, the smallest (bitrev3(rank mod 8), rank), where rank counts
+// the vertex's neighbour communities with a smaller id.
+__device__ __forceinline__ void nido_tie_slots(const MoveArgs& p, const Mass& m, const Table& t, int own, double ki,
+                                               double gm, unsigned long long& tk, int& cand) {
+  tk = kNoKey; cand = -1;
+  const int n = (int)t.mask + 1;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int cc = __ldcg(&t.keys[i]);
+    if (cc < 0 || cc == own) continue;
+    if (gain_of(__ldcg(&t.vals[i]), ki, p.a[cc], m) != gm) continue;
+    unsigned rank = 0;
+    for (int q = 0; q < n; ++q) {
+      const int kq = __ldcg(&t.keys[q]);
+      rank += (kq >= 0 && kq < cc) ? 1u : 0u;
     }
+    const unsigned long long key = nido_key(rank);
+    if (key < tk) { tk = key; cand = cc; }
   }
-  unsigned stage_parity = 0;
-  Table t;
-  if constexpr (kInts) {
-    t.slots = reinterpret_cast<unsigned long long*>(smem);
-    t.keys = nullptr;
-    t.vals = nullptr;
-    t.occ = reinterpret_cast<int*>(smem + kCap);
-    for (int i = threadIdx.x; i < kCap; i += kThreads) t.slots[i] = kEmptySlot;
-  } else {
-    t.vals = smem;
-    t.keys = reinterpret_cast<int*>(smem + kCap);
-    t.occ = kOcc ? t.keys + kCap : nullptr;
-    for (int i = threadIdx.x; i < kCap; i += kThreads) { t.keys[i] = -1; t.vals[i] = 0.; }
-  }
-  t.nocc = &nocc_s;
-  t.ints = kInts;
-  if (threadIdx.x == 0) nocc_s = 0;
-  __syncthreads();
-  const int wid = threadIdx.x >> 5;
-  // The next vertex's header (id, offsets, community, k, a_own) is loaded
-  // while the current one is evaluated, so its dependent round trips overlap.
-  int64_t task = blockIdx.x;
-  int v = 0, own = 0;
-  int64_t s = 0, eend = 0;
-  double ki = 0., aown = 0.;
-  if (task < n) {
-    v = list[task];
-    s = p.off[v];
-    eend = p.off[v + 1];
-    own = p.comm[v];
-    ki = p.k[v];
-    aown = p.a[own];
-  }
-  for (; task < n; task += gridDim.x) {
-    const int64_t nt = task + gridDim.x;
-    const int vn = nt < n ? list[nt] : 0;
-    int64_t sn = 0, en = 0;
-    if (nt < n) {
-      sn = p.off[vn];
-      en = p.off[vn + 1];
-    }
-    t.mask = min((unsigned)kCap, next_pow2_cap(eend - s)) - 1;
-    if constexpr (kStaged) {
-      if (!mbar_wait(&stage_bar, stage_parity)) atomicAdd(p.err, 1ull);
-      stage_parity ^= 1u;
-      accumulate_edges<true, 4>(p, v, s + (int64_t)wid * 32, eend, kThreads, t, sadj, sw, stage_off[0],
-                                stage_off[1]);
-    } else {
-      accumulate_edges<true, 4>(p, v, s + (int64_t)wid * 32, eend, kThreads, t);
-    }
-    __syncthreads();
-    if constexpr (kStaged) {
-      // every thread has read the stage (and stage_off): the next vertex's
-      // edges go into it while this one is evaluated
-      if (threadIdx.x == 0 && nt < n) {
-        int64_t a0, w0;
-        stage_edges(p, sn, en, sadj, sw, &stage_bar, &a0, &w0);
-        stage_off[0] = a0;
-        stage_off[1] = w0;
-      }
-    }
-    const int nu = kList ? nocc_s : (int)(t.mask + 1);
-    int ownn = 0;
-    double kin = 0.;
-    if (nt < n) {
-      ownn = p.comm[vn];
-      kin = p.k[vn];
-    }
-    // block_evaluate ends with a barrier that every thread reaches after
-    // reading nu, so the count can be reset right after it
-    block_evaluate(p, vertex_mass<kMulti>(p, v), t, nu, false, v, own, ki, aown, sg, stk, sc);
-    if (threadIdx.x == 0) nocc_s = 0;
-    const double aownn = nt < n ? p.a[ownn] : 0.;
-    for (int i = threadIdx.x; i < nu; i += kThreads) {
-      const int slot = kList ? t.occ[i] : i;
-      if constexpr (kInts) {
-        t.slots[slot] = kEmptySlot;
-      } else {
-        t.keys[slot] = -1;
-        t.vals[slot] = 0.;
-      }
-    }
-    __syncthreads();
-    v = vn;
-    s = sn;
-    eend = en;
-    own = ownn;
-    ki = kin;
-    aown = aownn;
-  }
+}
+
+// Evaluate a hub's filled table with the whole block under the reference's
+// tie rule and write newc[v].
+__device__ __forceinline__ void block_evaluate(const MoveArgs& p, const Mass& m, const Table& t, int v, int own,
+                                               double ki, double aown, double* sg, unsigned long long* stk, int* sc) {
+  double g = -NIDO_MAX_FLOAT, eown = 0.;
+  unsigned id = kNoId;
+  scan_slots(p, m, t, own, ki, eown, g, id);
+  eown = block_sum(eown, sg);  // nonzero in one thread at most: exact
+  const double gm = block_max(g, sg);
+  unsigned long long tk;
+  int cand;
+  nido_tie_slots(p, m, t, own, ki, gm, tk, cand);
+  g = cand >= 0 ? gm : -NIDO_MAX_FLOAT;
+  block_best(g, tk, cand, sg, stk, sc);
+  if (threadIdx.x == 0) decide(p, m, v, own, ki, aown, eown, g, (unsigned)cand);
 }
 
 // ---- degree > 2048: hub vertices split into segments of kHubSeg edges ----------
@@ -1065,13 +312,11 @@ __global__ void __launch_bounds__(kHubThreads) k_move_hub(const int2* __restrict
     Table t;
     t.keys = gkeys + hub_toff[h];
     t.vals = gvals + hub_toff[h];
-    t.occ = nullptr;
-    t.nocc = nullptr;
     t.mask = (unsigned)hub_cap[h] - 1;
     const int64_t s = p.off[v], eend = p.off[v + 1];
     const int64_t s0 = s + (int64_t)item.y * kHubSeg;
     const int64_t s1 = min(eend, s0 + kHubSeg);
-    accumulate_edges<true, 2, true>(p, v, s0 + (int64_t)wid * 32, s1, kHubThreads, t);
+    merge_edges_global<4>(p, v, s0 + (int64_t)wid * 32, s1, kHubThreads, t.keys, t.vals, t.mask);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last_s = atomicAdd(&hub_done[h], 1) == hub_nseg[h] - 1;
@@ -1080,7 +325,7 @@ __global__ void __launch_bounds__(kHubThreads) k_move_hub(const int2* __restrict
       __threadfence();
       const int own = p.comm[v];
       const double ki = p.k[v], aown = p.a[own];
-      block_evaluate(p, vertex_mass<kMulti>(p, v), t, (int)(t.mask + 1), true, v, own, ki, aown, sg, stk, sc);
+      block_evaluate(p, vertex_mass<kMulti>(p, v), t, v, own, ki, aown, sg, stk, sc);
       for (unsigned i = threadIdx.x; i <= t.mask; i += kHubThreads) {
         t.keys[i] = -1;
         t.vals[i] = 0.;
@@ -1289,7 +534,7 @@ __global__ void k_hub_combine(int64_t nh, const int32_t* __restrict__ hub_v, con
     if (lane == 0) {
       const int v = hub_v[h];
       const int own = p.comm[v];
-      decide(p, vertex_mass<kMulti>(p, v), v, own, p.k[v], p.a[own], eown, g, cand);
+      decide(p, vertex_mass<kMulti>(p, v), v, own, p.k[v], p.a[own], eown, g, (unsigned)cand);
     }
   }
 }
@@ -1455,7 +700,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_move_cluster(const int32_t* _
         be += re[r];
         if (better(rg[r], rtk[r], bg, bt)) { bg = rg[r]; bt = rtk[r]; bc = rc[r]; }
       }
-      decide(p, m, v, own, ki, aown, be, bg, bc);
+      decide(p, m, v, own, ki, aown, be, bg, (unsigned)bc);
     }
   }
 }
@@ -1628,83 +873,30 @@ int plan_hubs(nido_graph_s* g) {
   return NIDO_OK;
 }
 
-namespace {
-constexpr int kWarpCap = 256;     // warp tier: degree <= 128
-// threads per CTA and table slots of the CTA tiers
-constexpr int kCtaSThreads = 128;
-constexpr int kCtaMThreads = 256;
-constexpr int kCtaLThreads = 256;
-constexpr int kCtaSCap = 1024;
-constexpr int kCtaMCap = 2048;
-constexpr int kCtaLCap = 4096;
-// CTA-S and CTA-M with staged edges: table plus one vertex's widened ranges
-constexpr size_t smem_s_staged(bool ints) { return table_bytes(kCtaSCap, ints) + Stage<kCtaSMaxDeg>::kBytes; }
-constexpr size_t smem_m_staged(bool ints) { return table_bytes(kCtaMCap, ints) + Stage<kCtaMMaxDeg>::kBytes; }
-constexpr int kCtaXAThreads = 512;
-constexpr int kCtaXACap = 8192;   // 512-thread CTA-XA tier, two CTAs an SM (occupied list in integer phases)
-constexpr int kCtaXCap = 16384;   // 1024-thread CTA-XL tier (occupied list in integer phases)
-
-template <typename K>
-int set_smem(K kernel, size_t bytes) {
-  NIDO_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return NIDO_OK;
-}
-}  // namespace
 
 namespace {
-// CTAs of every move kernel that fit on the GPU at once (SMs x resident CTAs
-// per SM, from the occupancy calculator): grid-stride kernels launched with
-// more would leave a partial wave at the end.
-struct Resident {
-  int64_t g4 = kSMs, g8 = kSMs, g16 = kSMs, g32 = kSMs, warp = kSMs, ctas = kSMs, ctam = kSMs, ctal = kSMs,
-          ctaxa = kSMs, ctax = kSMs, hubmv = kSMs, hubins = kSMs, hubsl = kSMs, ctas_st = kSMs, ctam_st = kSMs;
+// CTAs of the hub kernels resident on the GPU at once, and of every tier
+// kernel (filled by TierKernels::init)
+struct HubResident {
+  int64_t mv = kSMs, ins = kSMs, sl = kSMs;
 };
-Resident g_resident[2][2];  // [many graphs][integer tables]
-
-template <typename K>
-int64_t resident(K kernel, int threads, size_t smem, int sms) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess) {
-    cudaGetLastError();
-    per_sm = 1;
-  }
-  return (int64_t)std::max(per_sm, 1) * sms;
-}
+HubResident g_hub_resident[2];      // [many graphs]
+TierResident g_resident[2][2][2];   // [many graphs][integer tables][reference tie rule]
 
 template <bool kMulti, bool kInts>
-int set_smem_mode() {
-  NIDO_TRY(set_smem(k_move_warp<kWarpCap, kMulti, kInts>, 8 * table_bytes(kWarpCap, kInts)));
-  NIDO_TRY(set_smem(k_move_cta<kCtaSThreads, kCtaSCap, kMulti, kInts>, table_bytes(kCtaSCap, kInts)));
-  NIDO_TRY(set_smem(k_move_cta<kCtaMThreads, kCtaMCap, kMulti, kInts>, table_bytes(kCtaMCap, kInts)));
-  NIDO_TRY(set_smem(k_move_cta<kCtaSThreads, kCtaSCap, kMulti, kInts, true, kCtaSMaxDeg>, smem_s_staged(kInts)));
-  NIDO_TRY(set_smem(k_move_cta<kCtaMThreads, kCtaMCap, kMulti, kInts, true, kCtaMMaxDeg>, smem_m_staged(kInts)));
-  NIDO_TRY(set_smem(k_move_cta<kCtaLThreads, kCtaLCap, kMulti, kInts>, table_bytes(kCtaLCap, kInts)));
-  NIDO_TRY(set_smem(k_move_cta<kCtaXAThreads, kCtaXACap, kMulti, kInts, false>, (size_t)kCtaXACap * 12));
-  NIDO_TRY(set_smem(k_move_cta<1024, kCtaXCap, kMulti, kInts, false>, (size_t)kCtaXCap * 12));
+int init_mode() {
   int dev = 0, sms = kSMs;
   NIDO_CUDA_TRY(cudaGetDevice(&dev));
   NIDO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   static std::mutex mu;  // contexts may be created from several threads
   std::lock_guard<std::mutex> lk(mu);
-  Resident& R = g_resident[kMulti ? 1 : 0][kInts ? 1 : 0];
-  R.g4 = resident(k_move_group<4, kMulti>, 256, 0, sms);
-  R.g8 = resident(k_move_group<8, kMulti>, 256, 0, sms);
-  R.g16 = resident(k_move_group<16, kMulti>, 256, 0, sms);
-  R.g32 = resident(k_move_group<32, kMulti>, 256, 0, sms);
-  R.warp = resident(k_move_warp<kWarpCap, kMulti, kInts>, 256, 8 * table_bytes(kWarpCap, kInts), sms);
-  R.ctas = resident(k_move_cta<kCtaSThreads, kCtaSCap, kMulti, kInts>, kCtaSThreads, table_bytes(kCtaSCap, kInts), sms);
-  R.ctam = resident(k_move_cta<kCtaMThreads, kCtaMCap, kMulti, kInts>, kCtaMThreads, table_bytes(kCtaMCap, kInts), sms);
-  R.ctas_st = resident(k_move_cta<kCtaSThreads, kCtaSCap, kMulti, kInts, true, kCtaSMaxDeg>, kCtaSThreads,
-                       smem_s_staged(kInts), sms);
-  R.ctam_st = resident(k_move_cta<kCtaMThreads, kCtaMCap, kMulti, kInts, true, kCtaMMaxDeg>, kCtaMThreads,
-                       smem_m_staged(kInts), sms);
-  R.ctal = resident(k_move_cta<kCtaLThreads, kCtaLCap, kMulti, kInts>, kCtaLThreads, table_bytes(kCtaLCap, kInts), sms);
-  R.ctaxa = resident(k_move_cta<kCtaXAThreads, kCtaXACap, kMulti, kInts, false>, kCtaXAThreads,
-                     (size_t)kCtaXACap * 12, sms);
-  R.ctax = resident(k_move_cta<1024, kCtaXCap, kMulti, kInts, false>, 1024, (size_t)kCtaXCap * 12, sms);
-  R.hubmv = resident(k_move_hub<kMulti>, kHubThreads, 0, sms);
-  R.hubins = resident(k_hub_insert, kHubThreads, 0, sms);
-  R.hubsl = resident(k_hub_slices<kMulti>, kHubThreads, 0, sms);
+  TierResident(&R)[2] = g_resident[kMulti ? 1 : 0][kInts ? 1 : 0];
+  NIDO_TRY((TierKernels<kMulti, kInts, false>::init(sms, &R[0])));
+  NIDO_TRY((TierKernels<kMulti, kInts, true>::init(sms, &R[1])));
+  HubResident& H = g_hub_resident[kMulti ? 1 : 0];
+  H.mv = resident_ctas(k_move_hub<kMulti>, kHubThreads, 0, sms);
+  H.ins = resident_ctas(k_hub_insert, kHubThreads, 0, sms);
+  H.sl = resident_ctas(k_hub_slices<kMulti>, kHubThreads, 0, sms);
   return NIDO_OK;
 }
 
@@ -1791,7 +983,9 @@ int launch_clusters(nido_graph_s* g, int batch, const MoveArgs& p, cudaStream_t 
 template <bool kMulti, bool kInts>
 int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
   nido_ctx_s* ctx = g->ctx;
-  const Resident& R = g_resident[kMulti ? 1 : 0][kInts ? 1 : 0];
+  const bool nido_tie = tie == NIDO_TIE_NIDO;
+  const TierResident& R = g_resident[kMulti ? 1 : 0][kInts ? 1 : 0][nido_tie ? 1 : 0];
+  const HubResident& H = g_hub_resident[kMulti ? 1 : 0];
   const cudaStream_t main_s = ctx->stream;
   NIDO_CUDA_TRY(cudaEventRecord(ctx->fork_ev, main_s));
   for (int i = 0; i < 2; ++i) NIDO_CUDA_TRY(cudaStreamWaitEvent(ctx->aux[i], ctx->fork_ev, 0));
@@ -1805,56 +999,17 @@ int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
     const int64_t n = b1 - b0;
     if (n <= 0) continue;
     const int32_t* list = g->perm + b0;
-    switch (t) {
-      case kTierG4:
-        k_move_group<4, kMulti><<<grid_cap((n + 63) / 64, R.g4), 256, 0, s>>>(list, n, p);
-        break;
-      case kTierG8:
-        k_move_group<8, kMulti><<<grid_cap((n + 31) / 32, R.g8), 256, 0, s>>>(list, n, p);
-        break;
-      case kTierG16:
-        k_move_group<16, kMulti><<<grid_cap((n + 15) / 16, R.g16), 256, 0, s>>>(list, n, p);
-        break;
-      case kTierG32:
-        k_move_group<32, kMulti><<<grid_cap((n + 7) / 8, R.g32), 256, 0, s>>>(list, n, p);
-        break;
-      case kTierWarp:
-        k_move_warp<kWarpCap, kMulti, kInts><<<grid_cap((n + 7) / 8, R.warp), 256, 8 * table_bytes(kWarpCap, kInts), s>>>(
-            list, n, p);
-        break;
-      case kTierCtaS:
-        if (staged)
-          k_move_cta<kCtaSThreads, kCtaSCap, kMulti, kInts, true, kCtaSMaxDeg>
-              <<<grid_cap(n, R.ctas_st), kCtaSThreads, smem_s_staged(kInts), s>>>(list, n, p);
-        else
-          k_move_cta<kCtaSThreads, kCtaSCap, kMulti, kInts>
-              <<<grid_cap(n, R.ctas), kCtaSThreads, table_bytes(kCtaSCap, kInts), s>>>(list, n, p);
-        break;
-      case kTierCtaM:
-        if (staged)
-          k_move_cta<kCtaMThreads, kCtaMCap, kMulti, kInts, true, kCtaMMaxDeg>
-              <<<grid_cap(n, R.ctam_st), kCtaMThreads, smem_m_staged(kInts), s>>>(list, n, p);
-        else
-          k_move_cta<kCtaMThreads, kCtaMCap, kMulti, kInts>
-              <<<grid_cap(n, R.ctam), kCtaMThreads, table_bytes(kCtaMCap, kInts), s>>>(list, n, p);
-        break;
-      case kTierCtaL:
-        k_move_cta<kCtaLThreads, kCtaLCap, kMulti, kInts><<<grid_cap(n, R.ctal), kCtaLThreads, table_bytes(kCtaLCap, kInts), s>>>(list, n, p);
-        break;
-      case kTierCtaXA:
-        k_move_cta<kCtaXAThreads, kCtaXACap, kMulti, kInts, false>
-            <<<grid_cap(n, R.ctaxa), kCtaXAThreads, (size_t)kCtaXACap * 12, s>>>(list, n, p);
-        break;
-      case kTierCtaX:
-        k_move_cta<1024, kCtaXCap, kMulti, kInts, false><<<grid_cap(n, R.ctax), 1024, (size_t)kCtaXCap * 12, s>>>(list, n, p);
-        break;
-      default: {
+    if (t != kTierHub) {
+      if (nido_tie) NIDO_TRY((TierKernels<kMulti, kInts, true>::launch(R, t, list, n, p, staged, s)));
+      else NIDO_TRY((TierKernels<kMulti, kInts, false>::launch(R, t, list, n, p, staged, s)));
+      continue;
+    }
         if constexpr (kInts) {
           // integer-weight phases with the smallest-id rule: hubs on
           // thread-block clusters when every hub of the phase fits one
           if (tie != NIDO_TIE_NIDO && g->cfg.hub_clusters && g->hub_cl_ok) {
             NIDO_TRY(launch_clusters<kMulti>(g, batch, p, s));
-            break;
+            continue;
           }
         }
         SliceResult* res = reinterpret_cast<SliceResult*>(g->hub_res);
@@ -1862,24 +1017,24 @@ int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
           const nido_graph_s::HubWave& w = g->hub_waves[wv];
           const int2* items = g->hub_items + w.i0;
           if (tie == NIDO_TIE_NIDO) {
-            k_move_hub<kMulti><<<grid_cap(w.i1 - w.i0, R.hubmv), kHubThreads, 0, s>>>(
+            k_move_hub<kMulti><<<grid_cap(w.i1 - w.i0, H.mv), kHubThreads, 0, s>>>(
                 items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, g->hub_nseg, g->hub_done, g->gkeys,
                 g->gvals, p);
             NIDO_LAUNCH_CHECK();
             continue;
           }
           if (kInts && g->gpacked && g->gslab_packed >= g->gslab_need) {
-            k_hub_insert_packed<<<grid_cap(w.i1 - w.i0, R.hubins), kHubThreads, 0, s>>>(
+            k_hub_insert_packed<<<grid_cap(w.i1 - w.i0, H.ins), kHubThreads, 0, s>>>(
                 items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, g->gpacked, p);
             NIDO_LAUNCH_CHECK();
-            k_hub_slices_packed<kMulti><<<grid_cap(w.s1 - w.s0, R.hubsl), kHubThreads, 0, s>>>(
+            k_hub_slices_packed<kMulti><<<grid_cap(w.s1 - w.s0, H.sl), kHubThreads, 0, s>>>(
                 g->hub_slices + w.s0, w.s1 - w.s0, g->hub_v, g->hub_toff, g->hub_capv, g->gpacked, p, res + w.s0);
             NIDO_LAUNCH_CHECK();
           } else {
-            k_hub_insert<<<grid_cap(w.i1 - w.i0, R.hubins), kHubThreads, 0, s>>>(
+            k_hub_insert<<<grid_cap(w.i1 - w.i0, H.ins), kHubThreads, 0, s>>>(
                 items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, g->gkeys, g->gvals, p);
             NIDO_LAUNCH_CHECK();
-            k_hub_slices<kMulti><<<grid_cap(w.s1 - w.s0, R.hubsl), kHubThreads, 0, s>>>(
+            k_hub_slices<kMulti><<<grid_cap(w.s1 - w.s0, H.sl), kHubThreads, 0, s>>>(
                 g->hub_slices + w.s0, w.s1 - w.s0, g->hub_v, g->hub_toff, g->hub_capv, g->gkeys, g->gvals, p,
                 res + w.s0);
             NIDO_LAUNCH_CHECK();
@@ -1888,10 +1043,6 @@ int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
               w.h1 - w.h0, g->hub_v + w.h0, g->hub_slice_first + w.h0, res, p);
           NIDO_LAUNCH_CHECK();
         }
-        continue;
-      }
-    }
-    NIDO_LAUNCH_CHECK();
   }
   for (int i = 0; i < 2; ++i) {
     NIDO_CUDA_TRY(cudaEventRecord(ctx->join_ev[i], ctx->aux[i]));
@@ -1903,10 +1054,10 @@ int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
 
 int move_init_attributes() {
   NIDO_TRY(cluster_init());
-  NIDO_TRY((set_smem_mode<false, false>()));
-  NIDO_TRY((set_smem_mode<false, true>()));
-  NIDO_TRY((set_smem_mode<true, false>()));
-  return set_smem_mode<true, true>();
+  NIDO_TRY((init_mode<false, false>()));
+  NIDO_TRY((init_mode<false, true>()));
+  NIDO_TRY((init_mode<true, false>()));
+  return init_mode<true, true>();
 }
 
 namespace {
