@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "engine.cuh"
+#include "hub_core.cuh"
 #include "move_core.cuh"
 #include "move_tiers.cuh"
 
@@ -49,461 +50,72 @@ __global__ void k_check_bounded_wait(int32_t* out) {
   out[1] = (int32_t)min((gtimer_ns() - t0) / 1000000ull, 1ull << 30);
 }
 
-// ---- hub tables in global memory ------------------------------------------------
-// Hub segments: the edges [first, eend) of vertex v in 32-edge chunks into a
-// global table; every lane keeps the compare-and-swaps of its kUnroll chunks in
-// flight together instead of finishing one chunk's probe before the next.
-// Equal communities within a chunk are still folded onto one lane first.
-template <int kUnroll>
-__device__ __forceinline__ void merge_edges_global(const MoveArgs& p, int v, int64_t first, int64_t eend,
-                                                   int64_t stride, int* keys, double* vals, unsigned mask) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t base = first; base < eend; base += kUnroll * stride) {
-    int u[kUnroll], c[kUnroll];
-    double wt[kUnroll];
-    unsigned h[kUnroll];
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      const int64_t j = base + k * stride + lane;
-      u[k] = -1;
-      wt[k] = 0.;
-      if (j < eend) {
-        u[k] = p.adj[j];
-        wt[k] = p.w[j];
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      c[k] = u[k] >= 0 ? p.comm[u[k]] : -1;
-      if (u[k] == v) wt[k] = 0.;
-    }
-    unsigned pending = 0u;
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      const bool ok = u[k] >= 0;
-      const unsigned peers = __match_any_sync(NIDO_FULL_MASK, c[k]);
-      wt[k] = fold_peers(peers, ok, wt[k]);
-      if (ok && lane == __ffs(peers) - 1) pending |= 1u << k;
-      h[k] = ok ? hash_slot(c[k], mask) : 0u;
-    }
-    for (unsigned probe = 0; pending != 0u && probe <= mask; ++probe) {
-      int old[kUnroll];
-#pragma unroll
-      for (int k = 0; k < kUnroll; ++k) old[k] = (pending >> k & 1u) ? atomicCAS(&keys[h[k]], -1, c[k]) : 0;
-#pragma unroll
-      for (int k = 0; k < kUnroll; ++k) {
-        if (!(pending >> k & 1u)) continue;
-        if (old[k] == -1 || old[k] == c[k]) {
-          atomicAdd(&vals[h[k]], wt[k]);
-          pending &= ~(1u << k);
-        } else {
-          h[k] = (h[k] + 1) & mask;
-        }
-      }
-    }
-    if (pending != 0u) atomicAdd(p.err, 1ull);
-  }
-}
-
-// merge_edges_global for packed integer tables (integer-weight phases): one
-// 64-bit slot per community (id, int32 sum), so a new community is one
-// compare-and-swap that also carries its first sum, an existing one one
-// 32-bit add.  Equal communities within a chunk are still folded onto one
-// lane first (fewer L2 atomics).
-template <int kUnroll>
-__device__ __forceinline__ void merge_edges_packed(const MoveArgs& p, int v, int64_t first, int64_t eend,
-                                                   int64_t stride, unsigned long long* slots, unsigned mask) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t base = first; base < eend; base += kUnroll * stride) {
-    int u[kUnroll], c[kUnroll], x[kUnroll];
-    double wt[kUnroll];
-    unsigned h[kUnroll];
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      const int64_t j = base + k * stride + lane;
-      u[k] = -1;
-      wt[k] = 0.;
-      if (j < eend) {
-        u[k] = p.adj[j];
-        wt[k] = p.w[j];
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      c[k] = u[k] >= 0 ? p.comm[u[k]] : -1;
-      if (u[k] == v) wt[k] = 0.;
-    }
-    unsigned pending = 0u;
-#pragma unroll
-    for (int k = 0; k < kUnroll; ++k) {
-      const bool ok = u[k] >= 0;
-      const unsigned peers = __match_any_sync(NIDO_FULL_MASK, c[k]);
-      x[k] = __double2int_rn(fold_peers(peers, ok, wt[k]));
-      if (ok && lane == __ffs(peers) - 1) pending |= 1u << k;
-      h[k] = ok ? hash_slot(c[k], mask) : 0u;
-    }
-    for (unsigned probe = 0; pending != 0u && probe <= mask; ++probe) {
-      unsigned long long old[kUnroll];
-#pragma unroll
-      for (int k = 0; k < kUnroll; ++k)
-        old[k] = (pending >> k & 1u)
-                     ? atomicCAS(&slots[h[k]], kEmptySlot, ((unsigned long long)(unsigned)c[k] << 32) | (unsigned)x[k])
-                     : 0ull;
-#pragma unroll
-      for (int k = 0; k < kUnroll; ++k) {
-        if (!(pending >> k & 1u)) continue;
-        if (old[k] == kEmptySlot) {
-          pending &= ~(1u << k);
-        } else if (slot_key(old[k]) == c[k]) {
-          atomicAdd(reinterpret_cast<int*>(&slots[h[k]]), x[k]);
-          pending &= ~(1u << k);
-        } else {
-          h[k] = (h[k] + 1) & mask;
-        }
-      }
-    }
-    if (pending != 0u) atomicAdd(p.err, 1ull);
-  }
-}
-
-// Block-wide argmax: every thread gets the result.
-__device__ void block_best(double& g, unsigned long long& tk, int& cand, double* sg,
-                           unsigned long long* stk, int* sc) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  group_best<32>(g, tk, cand);
-  if (lane == 0) { sg[wid] = g; stk[wid] = tk; sc[wid] = cand; }
-  __syncthreads();
-  if (wid == 0) {
-    g = lane < nw ? sg[lane] : -NIDO_MAX_FLOAT;
-    tk = lane < nw ? stk[lane] : kNoKey;
-    cand = lane < nw ? sc[lane] : -1;
-    group_best<32>(g, tk, cand);
-    if (lane == 0) { sg[0] = g; stk[0] = tk; sc[0] = cand; }
-  }
-  __syncthreads();
-  g = sg[0]; tk = stk[0]; cand = sc[0];
-  __syncthreads();
-}
-
-__device__ double block_sum(double x, double* sx) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  x = group_sum<32>(x);
-  if (lane == 0) sx[wid] = x;
-  __syncthreads();
-  double t = 0.;
-  for (int i = 0; i < nw; ++i) t += sx[i];
-  __syncthreads();
-  return t;
-}
-
-__device__ double block_max(double x, double* sx) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  x = group_max<32>(x);
-  if (lane == 0) sx[wid] = x;
-  __syncthreads();
-  double t = -NIDO_MAX_FLOAT;
-  for (int i = 0; i < nw; ++i) t = fmax(t, sx[i]);
-  __syncthreads();
-  return t;
-}
-
-// A hub's FP64 table (the reference's tie rule): cap = mask + 1 slots.
-struct Table {
-  int* keys;
-  double* vals;
-  unsigned mask;
-};
-
-// Scan the slots t0, t0+step, ... of a hub's table: e_own and the best (gain, id)
-// of this thread.  Slots are taken four at a time so that their a_c gathers are
-// in flight together.
-__device__ __forceinline__ void scan_slots(const MoveArgs& p, const Mass& m, const Table& t, int own, double ki,
-                                           double& eown, double& g, unsigned& id) {
-  constexpr int U = 4;
-  const int n = (int)t.mask + 1, step = (int)blockDim.x;
-  for (int i = threadIdx.x; i < n; i += U * step) {
-    int cc[U];
-    double val[U], ac[U];
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const int ii = i + k * step;
-      cc[k] = -1;
-      if (ii < n) {
-        cc[k] = __ldcg(&t.keys[ii]);
-        val[k] = __ldcg(&t.vals[ii]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < U; ++k) ac[k] = (cc[k] >= 0 && cc[k] != own) ? p.a[cc[k]] : 0.;
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      if (cc[k] < 0) continue;
-      if (cc[k] == own) {
-        eown = val[k];
-      } else {
-        const double gg = gain_of(val[k], ki, ac[k], m);
-        if (gg > g || (gg == g && (unsigned)cc[k] < id)) { g = gg; id = (unsigned)cc[k]; }
-      }
-    }
-  }
-}
-
-// The reference's tie rule over the same slots: among communities whose
-// gain equals gm, the smallest (bitrev3(rank mod 8), rank), where rank counts
-// the vertex's neighbour communities with a smaller id.
-__device__ __forceinline__ void nido_tie_slots(const MoveArgs& p, const Mass& m, const Table& t, int own, double ki,
-                                               double gm, unsigned long long& tk, int& cand) {
-  tk = kNoKey; cand = -1;
-  const int n = (int)t.mask + 1;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int cc = __ldcg(&t.keys[i]);
-    if (cc < 0 || cc == own) continue;
-    if (gain_of(__ldcg(&t.vals[i]), ki, p.a[cc], m) != gm) continue;
-    unsigned rank = 0;
-    for (int q = 0; q < n; ++q) {
-      const int kq = __ldcg(&t.keys[q]);
-      rank += (kq >= 0 && kq < cc) ? 1u : 0u;
-    }
-    const unsigned long long key = nido_key(rank);
-    if (key < tk) { tk = key; cand = cc; }
-  }
-}
-
-// Evaluate a hub's filled table with the whole block under the reference's
-// tie rule and write newc[v].
-__device__ __forceinline__ void block_evaluate(const MoveArgs& p, const Mass& m, const Table& t, int v, int own,
-                                               double ki, double aown, double* sg, unsigned long long* stk, int* sc) {
-  double g = -NIDO_MAX_FLOAT, eown = 0.;
-  unsigned id = kNoId;
-  scan_slots(p, m, t, own, ki, eown, g, id);
-  eown = block_sum(eown, sg);  // nonzero in one thread at most: exact
-  const double gm = block_max(g, sg);
-  unsigned long long tk;
-  int cand;
-  nido_tie_slots(p, m, t, own, ki, gm, tk, cand);
-  g = cand >= 0 ? gm : -NIDO_MAX_FLOAT;
-  block_best(g, tk, cand, sg, stk, sc);
-  if (threadIdx.x == 0) decide(p, m, v, own, ki, aown, eown, g, (unsigned)cand);
-}
-
-// ---- degree > 2048: hub vertices split into segments of kHubSeg edges ----------
-// Each CTA takes one (hub, segment) item and merges its edges into the hub's
-// table in global memory (L2-resident); the CTA that finishes a hub's last
-// segment (an atomic ticket; nobody waits) evaluates and clears the table.
-constexpr int kHubThreads = 256;
-
-template <bool kMulti>
+// ---- hubs: segments of kHubSeg edges, tables in global memory ----------------------
+// The reference's tie rule: each CTA takes one (hub, segment) item and merges
+// its edges into the hub's table; the CTA that finishes a hub's last segment (an
+// atomic ticket; nobody waits) evaluates and clears the table.
+template <bool kMulti, bool kInts>
 __global__ void __launch_bounds__(kHubThreads) k_move_hub(const int2* __restrict__ items, int64_t n,
                                                           const int32_t* __restrict__ hub_v,
                                                           const int64_t* __restrict__ hub_toff,
                                                           const int32_t* __restrict__ hub_cap,
                                                           const int32_t* __restrict__ hub_nseg,
-                                                          int32_t* __restrict__ hub_done, int32_t* gkeys,
-                                                          double* gvals, MoveArgs p) {
-  __shared__ double sg[32];
-  __shared__ unsigned long long stk[32];
-  __shared__ int sc[32];
+                                                          int32_t* __restrict__ hub_done, HubTable<kInts> tab,
+                                                          MoveArgs p) {
+  __shared__ HubShared sh;
+  __shared__ TieShared ts;
   __shared__ int last_s;
-  const int wid = threadIdx.x >> 5;
   for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {
     const int2 item = items[it];
     const int h = item.x;
     const int v = hub_v[h];
-    Table t;
-    t.keys = gkeys + hub_toff[h];
-    t.vals = gvals + hub_toff[h];
-    t.mask = (unsigned)hub_cap[h] - 1;
-    const int64_t s = p.off[v], eend = p.off[v + 1];
-    const int64_t s0 = s + (int64_t)item.y * kHubSeg;
-    const int64_t s1 = min(eend, s0 + kHubSeg);
-    merge_edges_global<4>(p, v, s0 + (int64_t)wid * 32, s1, kHubThreads, t.keys, t.vals, t.mask);
+    const HubTable<kInts> t = tab.at(hub_toff[h]);
+    hub_segment<kInts>(p, v, item.y, t, hub_cap[h]);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last_s = atomicAdd(&hub_done[h], 1) == hub_nseg[h] - 1;
     __syncthreads();
     if (last_s) {
       __threadfence();
-      const int own = p.comm[v];
-      const double ki = p.k[v], aown = p.a[own];
-      block_evaluate(p, vertex_mass<kMulti>(p, v), t, v, own, ki, aown, sg, stk, sc);
-      for (unsigned i = threadIdx.x; i <= t.mask; i += kHubThreads) {
-        t.keys[i] = -1;
-        t.vals[i] = 0.;
-      }
+      hub_tie<kMulti, kInts>(p, v, t, hub_cap[h], sh, ts);
       if (threadIdx.x == 0) hub_done[h] = 0;
     }
     __syncthreads();
   }
 }
 
-// Fast path for the smallest-id rule: segments only merge (k_hub_insert),
-// then every kHubSlice-slot slice of a table is scanned and cleared by its
-// own CTA (k_hub_slices), and one warp per hub combines the slice results
-// (k_hub_combine).  The reference's tie rule needs ranks over the whole
-// table and uses k_move_hub instead.
-constexpr int kHubSlice = 4096;
-// The table slots of one wave of hubs come from the graph's tier
-// configuration (default 4M slots: 48 MB of keys and values, which leaves
+// The smallest-id rule: segments only merge (k_hub_insert), then every
+// kHubSlice-slot slice of a table is scanned and cleared by its own CTA
+// (k_hub_slices), and one warp per hub combines the slice results
+// (k_hub_combine).  The table slots of one wave of hubs come from the graph's
+// tier configuration (default 4M slots: 48 MB of keys and values, which leaves
 // room in the 126 MB L2 for the streamed adjacency and the gathers).
-
+template <bool kInts>
 __global__ void __launch_bounds__(kHubThreads) k_hub_insert(const int2* __restrict__ items, int64_t n,
                                                             const int32_t* __restrict__ hub_v,
                                                             const int64_t* __restrict__ hub_toff,
-                                                            const int32_t* __restrict__ hub_cap, int32_t* gkeys,
-                                                            double* gvals, MoveArgs p) {
-  const int wid = threadIdx.x >> 5;
+                                                            const int32_t* __restrict__ hub_cap, HubTable<kInts> tab,
+                                                            MoveArgs p) {
   for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {
     const int2 item = items[it];
     const int h = item.x;
-    const int v = hub_v[h];
-    const int64_t s = p.off[v], eend = p.off[v + 1];
-    const int64_t s0 = s + (int64_t)item.y * kHubSeg;
-    merge_edges_global<4>(p, v, s0 + (int64_t)wid * 32, min(eend, s0 + kHubSeg), kHubThreads, gkeys + hub_toff[h],
-                          gvals + hub_toff[h], (unsigned)hub_cap[h] - 1);
+    hub_segment<kInts>(p, hub_v[h], item.y, tab.at(hub_toff[h]), hub_cap[h]);
   }
 }
 
-struct SliceResult {
-  double g;
-  double eown;
-  unsigned long long tk;
-  int cand;
-  int pad;
-};
-
-// Slice y of hub x covers slots [y*kHubSlice, (y+1)*kHubSlice) of the hub's
-// table, read and cleared in order.  (A per-hub list of occupied slots,
-// appended during the merge, measured twice as slow on R-MAT scale 22: the
-// hub tables are mostly full and the list's counter is one contended
-// address per hub.)
-template <bool kMulti>
+template <bool kMulti, bool kInts>
 __global__ void __launch_bounds__(kHubThreads) k_hub_slices(const int2* __restrict__ slices, int64_t n,
                                                             const int32_t* __restrict__ hub_v,
                                                             const int64_t* __restrict__ hub_toff,
-                                                            const int32_t* __restrict__ hub_cap, int32_t* gkeys,
-                                                            double* gvals, MoveArgs p,
-                                                            SliceResult* __restrict__ res) {
-  __shared__ double sg[32];
-  __shared__ unsigned long long stk[32];
-  __shared__ int sc[32];
+                                                            const int32_t* __restrict__ hub_cap, HubTable<kInts> tab,
+                                                            MoveArgs p, SliceResult* __restrict__ res) {
+  __shared__ HubShared sh;
   for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {
     const int2 sl = slices[it];
     const int len = min(kHubSlice, hub_cap[sl.x] - sl.y * kHubSlice);
-    const int v = hub_v[sl.x];
-    int* keys = gkeys + hub_toff[sl.x] + (int64_t)sl.y * kHubSlice;
-    double* vals = gvals + hub_toff[sl.x] + (int64_t)sl.y * kHubSlice;
-    const int own = p.comm[v];
-    const double ki = p.k[v];
-    const Mass m = vertex_mass<kMulti>(p, v);
-    double g = -NIDO_MAX_FLOAT, eown = 0.;
-    unsigned long long tk = kNoKey;
-    int cand = -1;
-    // four slots per thread at a time, so their a_c gathers are in flight together
-    constexpr int U = 4;
-    for (int i0 = threadIdx.x; i0 < len; i0 += U * kHubThreads) {
-      int cc[U];
-      double val[U], ac[U];
-#pragma unroll
-      for (int k = 0; k < U; ++k) {
-        const int i = i0 + k * kHubThreads;
-        cc[k] = -1;
-        if (i < len) {
-          cc[k] = keys[i];
-          val[k] = vals[i];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < U; ++k) ac[k] = (cc[k] >= 0 && cc[k] != own) ? p.a[cc[k]] : 0.;
-#pragma unroll
-      for (int k = 0; k < U; ++k) {
-        if (cc[k] < 0) continue;
-        const int i = i0 + k * kHubThreads;
-        keys[i] = -1;
-        vals[i] = 0.;
-        if (cc[k] == own) {
-          eown = val[k];
-        } else {
-          const double gg = gain_of(val[k], ki, ac[k], m);
-          if (better(gg, (unsigned)cc[k], g, tk)) { g = gg; tk = (unsigned)cc[k]; cand = cc[k]; }
-        }
-      }
-    }
-    eown = block_sum(eown, sg);
-    block_best(g, tk, cand, sg, stk, sc);
-    if (threadIdx.x == 0) res[it] = SliceResult{g, eown, tk, cand, 0};
-  }
-}
-
-// k_hub_insert / k_hub_slices on packed integer tables
-__global__ void __launch_bounds__(kHubThreads) k_hub_insert_packed(const int2* __restrict__ items, int64_t n,
-                                                                   const int32_t* __restrict__ hub_v,
-                                                                   const int64_t* __restrict__ hub_toff,
-                                                                   const int32_t* __restrict__ hub_cap,
-                                                                   unsigned long long* gslots, MoveArgs p) {
-  const int wid = threadIdx.x >> 5;
-  for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {
-    const int2 item = items[it];
-    const int h = item.x;
-    const int v = hub_v[h];
-    const int64_t s = p.off[v], eend = p.off[v + 1];
-    const int64_t s0 = s + (int64_t)item.y * kHubSeg;
-    merge_edges_packed<4>(p, v, s0 + (int64_t)wid * 32, min(eend, s0 + kHubSeg), kHubThreads, gslots + hub_toff[h],
-                          (unsigned)hub_cap[h] - 1);
-  }
-}
-
-template <bool kMulti>
-__global__ void __launch_bounds__(kHubThreads) k_hub_slices_packed(const int2* __restrict__ slices, int64_t n,
-                                                                   const int32_t* __restrict__ hub_v,
-                                                                   const int64_t* __restrict__ hub_toff,
-                                                                   const int32_t* __restrict__ hub_cap,
-                                                                   unsigned long long* gslots, MoveArgs p,
-                                                                   SliceResult* __restrict__ res) {
-  __shared__ double sg[32];
-  __shared__ unsigned long long stk[32];
-  __shared__ int sc[32];
-  for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {
-    const int2 sl = slices[it];
-    const int len = min(kHubSlice, hub_cap[sl.x] - sl.y * kHubSlice);
-    const int v = hub_v[sl.x];
-    unsigned long long* slots = gslots + hub_toff[sl.x] + (int64_t)sl.y * kHubSlice;
-    const int own = p.comm[v];
-    const double ki = p.k[v];
-    const Mass m = vertex_mass<kMulti>(p, v);
-    double g = -NIDO_MAX_FLOAT, eown = 0.;
-    unsigned long long tk = kNoKey;
-    int cand = -1;
-    constexpr int U = 4;
-    for (int i0 = threadIdx.x; i0 < len; i0 += U * kHubThreads) {
-      int cc[U];
-      double val[U], ac[U];
-#pragma unroll
-      for (int k = 0; k < U; ++k) {
-        const int i = i0 + k * kHubThreads;
-        cc[k] = -1;
-        if (i < len) {
-          const unsigned long long x = __ldcg(&slots[i]);
-          cc[k] = slot_key(x);
-          val[k] = (double)slot_sum(x);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < U; ++k) ac[k] = (cc[k] >= 0 && cc[k] != own) ? p.a[cc[k]] : 0.;
-#pragma unroll
-      for (int k = 0; k < U; ++k) {
-        if (cc[k] < 0) continue;
-        slots[i0 + k * kHubThreads] = kEmptySlot;
-        if (cc[k] == own) {
-          eown = val[k];
-        } else {
-          const double gg = gain_of(val[k], ki, ac[k], m);
-          if (better(gg, (unsigned)cc[k], g, tk)) { g = gg; tk = (unsigned)cc[k]; cand = cc[k]; }
-        }
-      }
-    }
-    eown = block_sum(eown, sg);
-    block_best(g, tk, cand, sg, stk, sc);
-    if (threadIdx.x == 0) res[it] = SliceResult{g, eown, tk, cand, 0};
+    const SliceResult r =
+        hub_slice<kMulti, kInts>(p, hub_v[sl.x], tab.at(hub_toff[sl.x] + (int64_t)sl.y * kHubSlice), len, sh);
+    if (threadIdx.x == 0) res[it] = r;
   }
 }
 
@@ -515,27 +127,11 @@ __global__ void k_fill_u64(unsigned long long* __restrict__ x, int64_t n, unsign
 template <bool kMulti>
 __global__ void k_hub_combine(int64_t nh, const int32_t* __restrict__ hub_v, const int64_t* __restrict__ slice_first,
                               const SliceResult* __restrict__ res, MoveArgs p) {
-  const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t h = warp; h < nh; h += nw) {
     const int64_t r0 = slice_first[h], r1 = slice_first[h + 1];
-    if (r1 == r0) continue;  // hub of another batch
-    double g = -NIDO_MAX_FLOAT, eown = 0.;
-    unsigned long long tk = kNoKey;
-    int cand = -1;
-    for (int64_t r = r0 + lane; r < r1; r += 32) {
-      const SliceResult x = res[r];
-      eown += x.eown;
-      if (better(x.g, x.tk, g, tk)) { g = x.g; tk = x.tk; cand = x.cand; }
-    }
-    eown = group_sum<32>(eown);
-    group_best<32>(g, tk, cand);
-    if (lane == 0) {
-      const int v = hub_v[h];
-      const int own = p.comm[v];
-      decide(p, vertex_mass<kMulti>(p, v), v, own, p.k[v], p.a[own], eown, g, (unsigned)cand);
-    }
+    if (r1 > r0) hub_combine<kMulti>(p, hub_v[h], res + r0, r1 - r0);  // else a hub of another batch
   }
 }
 
@@ -819,7 +415,9 @@ int plan_hubs(nido_graph_s* g) {
   NIDO_CUDA_TRY(cudaMemcpyAsync(g->hub_item_first, ifirst.data(), sizeof(int64_t) * (nh + 1), cudaMemcpyHostToDevice, s));
   NIDO_CUDA_TRY(cudaMemcpyAsync(g->hub_slices, slices.data(), sizeof(int2) * slices.size(), cudaMemcpyHostToDevice, s));
   NIDO_CUDA_TRY(cudaMemcpyAsync(g->hub_slice_first, sfirst.data(), sizeof(int64_t) * (nh + 1), cudaMemcpyHostToDevice, s));
-  if (toff > g->gslab) {
+  // FP64 tables, or packed ones in integer-weight phases; both are kept empty
+  // between waves by the kernels that evaluate them
+  if (!g->int_weights && toff > g->gslab) {
     raw_free(g->ctx, g->gkeys);
     raw_free(g->ctx, g->gvals);
     g->gkeys = nullptr;
@@ -831,8 +429,6 @@ int plan_hubs(nido_graph_s* g) {
     NIDO_CUDA_TRY(cudaMemsetAsync(g->gvals, 0, sizeof(double) * (size_t)toff, s));
     g->gslab = toff;
   }
-  // packed tables for integer-weight phases (smallest-id rule), kept empty
-  // between waves by the slice scans like the FP64 ones
   if (g->int_weights && toff > g->gslab_packed) {
     raw_free(g->ctx, g->gpacked);
     g->gpacked = nullptr;
@@ -880,7 +476,7 @@ namespace {
 struct HubResident {
   int64_t mv = kSMs, ins = kSMs, sl = kSMs;
 };
-HubResident g_hub_resident[2];      // [many graphs]
+HubResident g_hub_resident[2][2];   // [many graphs][integer tables]
 TierResident g_resident[2][2][2];   // [many graphs][integer tables][reference tie rule]
 
 template <bool kMulti, bool kInts>
@@ -893,10 +489,10 @@ int init_mode() {
   TierResident(&R)[2] = g_resident[kMulti ? 1 : 0][kInts ? 1 : 0];
   NIDO_TRY((TierKernels<kMulti, kInts, false>::init(sms, &R[0])));
   NIDO_TRY((TierKernels<kMulti, kInts, true>::init(sms, &R[1])));
-  HubResident& H = g_hub_resident[kMulti ? 1 : 0];
-  H.mv = resident_ctas(k_move_hub<kMulti>, kHubThreads, 0, sms);
-  H.ins = resident_ctas(k_hub_insert, kHubThreads, 0, sms);
-  H.sl = resident_ctas(k_hub_slices<kMulti>, kHubThreads, 0, sms);
+  HubResident& H = g_hub_resident[kMulti ? 1 : 0][kInts ? 1 : 0];
+  H.mv = resident_ctas(k_move_hub<kMulti, kInts>, kHubThreads, 0, sms);
+  H.ins = resident_ctas(k_hub_insert<kInts>, kHubThreads, 0, sms);
+  H.sl = resident_ctas(k_hub_slices<kMulti, kInts>, kHubThreads, 0, sms);
   return NIDO_OK;
 }
 
@@ -985,7 +581,7 @@ int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
   nido_ctx_s* ctx = g->ctx;
   const bool nido_tie = tie == NIDO_TIE_NIDO;
   const TierResident& R = g_resident[kMulti ? 1 : 0][kInts ? 1 : 0][nido_tie ? 1 : 0];
-  const HubResident& H = g_hub_resident[kMulti ? 1 : 0];
+  const HubResident& H = g_hub_resident[kMulti ? 1 : 0][kInts ? 1 : 0];
   const cudaStream_t main_s = ctx->stream;
   NIDO_CUDA_TRY(cudaEventRecord(ctx->fork_ev, main_s));
   for (int i = 0; i < 2; ++i) NIDO_CUDA_TRY(cudaStreamWaitEvent(ctx->aux[i], ctx->fork_ev, 0));
@@ -1013,32 +609,24 @@ int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
           }
         }
         SliceResult* res = reinterpret_cast<SliceResult*>(g->hub_res);
+        HubTable<kInts> tab;
+        if constexpr (kInts) tab.slots = g->gpacked;  // integer phases are planned with packed tables
+        else tab = HubTable<false>{g->gkeys, g->gvals};
         for (int64_t wv = g->hub_wave_off[batch]; wv < g->hub_wave_off[batch + 1]; ++wv) {
           const nido_graph_s::HubWave& w = g->hub_waves[wv];
           const int2* items = g->hub_items + w.i0;
-          if (tie == NIDO_TIE_NIDO) {
-            k_move_hub<kMulti><<<grid_cap(w.i1 - w.i0, H.mv), kHubThreads, 0, s>>>(
-                items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, g->hub_nseg, g->hub_done, g->gkeys,
-                g->gvals, p);
+          if (nido_tie) {
+            k_move_hub<kMulti, kInts><<<grid_cap(w.i1 - w.i0, H.mv), kHubThreads, 0, s>>>(
+                items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, g->hub_nseg, g->hub_done, tab, p);
             NIDO_LAUNCH_CHECK();
             continue;
           }
-          if (kInts && g->gpacked && g->gslab_packed >= g->gslab_need) {
-            k_hub_insert_packed<<<grid_cap(w.i1 - w.i0, H.ins), kHubThreads, 0, s>>>(
-                items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, g->gpacked, p);
-            NIDO_LAUNCH_CHECK();
-            k_hub_slices_packed<kMulti><<<grid_cap(w.s1 - w.s0, H.sl), kHubThreads, 0, s>>>(
-                g->hub_slices + w.s0, w.s1 - w.s0, g->hub_v, g->hub_toff, g->hub_capv, g->gpacked, p, res + w.s0);
-            NIDO_LAUNCH_CHECK();
-          } else {
-            k_hub_insert<<<grid_cap(w.i1 - w.i0, H.ins), kHubThreads, 0, s>>>(
-                items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, g->gkeys, g->gvals, p);
-            NIDO_LAUNCH_CHECK();
-            k_hub_slices<kMulti><<<grid_cap(w.s1 - w.s0, H.sl), kHubThreads, 0, s>>>(
-                g->hub_slices + w.s0, w.s1 - w.s0, g->hub_v, g->hub_toff, g->hub_capv, g->gkeys, g->gvals, p,
-                res + w.s0);
-            NIDO_LAUNCH_CHECK();
-          }
+          k_hub_insert<kInts><<<grid_cap(w.i1 - w.i0, H.ins), kHubThreads, 0, s>>>(
+              items, w.i1 - w.i0, g->hub_v, g->hub_toff, g->hub_capv, tab, p);
+          NIDO_LAUNCH_CHECK();
+          k_hub_slices<kMulti, kInts><<<grid_cap(w.s1 - w.s0, H.sl), kHubThreads, 0, s>>>(
+              g->hub_slices + w.s0, w.s1 - w.s0, g->hub_v, g->hub_toff, g->hub_capv, tab, p, res + w.s0);
+          NIDO_LAUNCH_CHECK();
           k_hub_combine<kMulti><<<grid_cap((w.h1 - w.h0 + 7) / 8, kSMs * 4), 256, 0, s>>>(
               w.h1 - w.h0, g->hub_v + w.h0, g->hub_slice_first + w.h0, res, p);
           NIDO_LAUNCH_CHECK();
@@ -1061,10 +649,10 @@ int move_init_attributes() {
 }
 
 namespace {
-MoveArgs move_args(nido_graph_s* g, int tie) {
+MoveArgs move_args(nido_graph_s* g) {
   double zh = 0., zl = 0.;
   if (!g->gid && g->int_weights) mass_reciprocal(g->m, &zh, &zl);
-  return MoveArgs{g->off, g->adj, g->w, g->comm, g->k, g->a, g->newc, g->m, tie,
+  return MoveArgs{g->off, g->adj, g->w, g->comm, g->k, g->a, g->newc, g->m,
                   reinterpret_cast<unsigned long long*>(g->dcount + 1), g->gid, g->mg, zh, zl,
                   g->int_weights ? g->zg : nullptr,
                   g->int_weights ? 1 : 0, g->nv};
@@ -1082,7 +670,7 @@ int tiers_direct(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
 int launch_move_tiers(nido_graph_s* g, int batch, int tie) {
   if (batch < 0 || batch >= g->nbatches)
     return nido_set_error(NIDO_E_INVALID, "louvain_update: batch %d out of range [0,%d)", batch, g->nbatches);
-  return tiers_direct(g, batch, tie, move_args(g, tie));
+  return tiers_direct(g, batch, tie, move_args(g));
 }
 
 int check_bounded_wait(nido_ctx_s* ctx, int32_t* gave_up, int32_t* waited_ms) {
@@ -1106,7 +694,7 @@ int launch_move(nido_graph_s* g, int batch, int tie, cudaEvent_t ev_start, cudaE
     return nido_set_error(NIDO_E_INVALID, "louvain_update: batch %d out of range [0,%d)", batch, g->nbatches);
   if (!g->bins_valid) NIDO_TRY(build_batches(g));
   cudaStream_t s = g->ctx->stream;
-  const MoveArgs p = move_args(g, tie);
+  const MoveArgs p = move_args(g);
   if (ev_start) NIDO_CUDA_TRY(cudaEventRecord(ev_start, s));
   auto direct = [&]() { return tiers_direct(g, batch, tie, p); };
   if (!g->use_graphs) {

@@ -20,7 +20,6 @@ struct MoveArgs {
   const double* __restrict__ a;
   int32_t* __restrict__ newc;
   double m;
-  int tie;
   unsigned long long* err;  // probe-limit failures (never expected)
   // many-graph mode: graph of every vertex and mass of every graph (null for
   // one graph, whose mass is m)
