@@ -79,6 +79,14 @@ namespace nido {
 namespace {
 
 constexpr int kThreads = 256;
+// The persistent loop stops to drop stopped graphs from the tier lists when the
+// iterating graphs hold fewer than this many of listed_v vertices.  Listing
+// again costs the host some 150 us, about two sweeps of a million edges, so
+// small lists wait for a quarter and the smallest are swept to the end.
+int64_t relist_below(int64_t listed_v, int64_t listed_e) {
+  if (listed_e > (int64_t)4 << 20) return (3 * listed_v + 3) / 4;
+  return listed_e > (int64_t)128 << 10 ? listed_v / 4 : 0;
+}
 
 inline unsigned grid_for(int64_t work, int per_block, int max_blocks = kSMs * 16) {
   int64_t b = (work + per_block - 1) / per_block;
@@ -494,10 +502,12 @@ int batch_modularity(nido_batch_s* B, const Lists& ql, double* out) {
 // in ids, which become the listed (gactive) graphs
 // The graphs ids are listed: modularity groups, active flags and the tier
 // lists of their vertices.  relist: ids is a subset of the graphs listed so
-// far in this phase, so the tier lists are compacted instead of rebuilt.
-int batch_list(nido_batch_s* B, const std::vector<int32_t>& ids, const std::vector<int64_t>& base, Lists* ql,
-               bool relist = false) {
+// far in this phase, so the tier lists are compacted instead of rebuilt (unless
+// their edges became few enough for the persistent phase loop).
+int batch_list(nido_batch_s* B, const std::vector<int32_t>& ids, const std::vector<int64_t>& base, int64_t edges,
+               Lists* ql, bool relist = false) {
   nido_graph_s* g = B->g;
+  g->plan_ne = edges;
   cudaStream_t s = g->ctx->stream;
   NIDO_CUDA_TRY(cudaMemsetAsync(B->gactive, 0, sizeof(int32_t) * B->ng, s));
   *ql = make_list(ids, base, q_groups);
@@ -507,7 +517,7 @@ int batch_list(nido_batch_s* B, const std::vector<int32_t>& ids, const std::vect
     NIDO_LAUNCH_CHECK();
   }
   if (ql->off.back() > B->cap_modv) return nido_set_error(NIDO_E_NOMEM, "modularity buffer too small");
-  if (relist && g->bins_valid) return compact_batches(g);
+  if (relist && g->bins_valid && (g->loop_plan || !loop_plan_fits(g, g->nbatches))) return compact_batches(g);
   g->bins_valid = false;
   return build_batches(g);
 }
@@ -572,6 +582,9 @@ extern "C" int nido_batch_upload(nido_ctx ctx, int32_t ngraphs, const int64_t* v
     return nido_set_error(NIDO_E_INVALID, "vertex bases must run from 0 to nv");
   for (int32_t i = 0; i < ngraphs; ++i)
     if (vbase[i + 1] < vbase[i]) return nido_set_error(NIDO_E_INVALID, "vertex bases must not decrease");
+  NIDO_CUDA_TRY(cudaSetDevice(ctx->device));
+  NIDO_TRY(move_init_attributes(true));
+  NIDO_TRY(phase_loop_init(true));
   nido_graph g = nullptr;
   NIDO_TRY(nido_graph_upload(ctx, nv, ne, off, adj, w, nbatches, &g));
   nido_batch B = new (std::nothrow) nido_batch_s();
@@ -737,7 +750,7 @@ extern "C" int nido_batch_run(nido_batch B, const nido_params* p, int64_t* out_c
     NIDO_LAUNCH_CHECK();
     NIDO_CUDA_TRY(cudaMemcpyAsync(edges.data(), B->gedges, sizeof(int64_t) * ng, cudaMemcpyDeviceToHost, s));
     Lists ql;
-    NIDO_TRY(batch_list(B, act, base, &ql));  // synchronizes
+    NIDO_TRY(batch_list(B, act, base, g->ne, &ql));  // synchronizes
     int64_t listed_v = 0, listed_e = 0;
     for (int32_t i : act) { listed_v += base[i + 1] - base[i]; listed_e += edges[i]; }
     // singleton start and Q_old (the tier autotuner, when asked, times move
@@ -754,11 +767,39 @@ extern "C" int nido_batch_run(nido_batch B, const nido_params* p, int64_t* out_c
       k_set_flags<<<grid_for(np, kThreads), kThreads, 0, s>>>(B->plist, np, B->giter);
       NIDO_LAUNCH_CHECK();
     }
-    NIDO_TRY(batch_modularity(B, ql, B->Q));
-    NIDO_CUDA_TRY(cudaMemcpyAsync(B->Qold, B->Q, sizeof(double) * ng, cudaMemcpyDeviceToDevice, s));
+    // Sweeps on the persistent kernel, which small phases (and the few graphs left
+    // of a large one) run on by default: until no graph iterates, or until enough
+    // stopped that listing the others again pays.
+    auto persistent_sweeps = [&](bool with_q, bool* unsupported) -> int {
+      LoopGraphs L{B->llist, B->qoff, (int)ql.ids.size(), ql.nbig, B->modv, B->Q, with_q ? B->Qold : nullptr,
+                   B->loops_phase, B->loops_total, B->giter, B->grest, relist_below(listed_v, listed_e)};
+      PhaseLoop r;
+      NIDO_TRY(persistent_phase_loop(g, p->tie_mode, tau, p->max_iter, false, &L, &r, unsupported));
+      if (*unsupported) return NIDO_OK;
+      NIDO_CUDA_TRY(cudaMemsetAsync(B->grest, 0, sizeof(int32_t) * ng, s));
+      st.move_launches += (int64_t)nb * r.loops;
+      st.edges_scanned += (double)listed_e * (double)r.loops;
+      st.move_bytes += (16.0 * (double)listed_e + 32.0 * (double)listed_vertices(g)) * (double)r.loops;
+      st.total_loops += r.loops;
+      st.move_ms += r.move_ms;
+      st.q_ms += r.q_ms;
+      for (int i = 0; i < 4; ++i) cnt[i] = r.counters[i];
+      return NIDO_OK;
+    };
+    int64_t n_iter = p->max_iter > 0 ? np : 0;
+    bool swept = false;  // the first sweeps ran (with Q and Qold) on the persistent kernel
+    if (p->host_loop == 0 && n_iter > 0 && g->loop_plan) {
+      bool unsupported = false;
+      NIDO_TRY(persistent_sweeps(true, &unsupported));
+      swept = !unsupported;
+      if (swept) n_iter = (int64_t)cnt[0];
+    }
+    if (!swept) {
+      NIDO_TRY(batch_modularity(B, ql, B->Q));
+      NIDO_CUDA_TRY(cudaMemcpyAsync(B->Qold, B->Q, sizeof(double) * ng, cudaMemcpyDeviceToDevice, s));
+    }
     NIDO_CUDA_TRY(cudaStreamSynchronize(s));
     lap(4);
-    int64_t n_iter = p->max_iter > 0 ? np : 0;
     // the commit of every batch's listed vertices of the iterating graphs
     auto commit_batch = [&](int b) -> int {
       PermRanges r{};
@@ -872,9 +913,13 @@ extern "C" int nido_batch_run(nido_batch B, const nido_params* p, int64_t* out_c
       return NIDO_OK;
     };
     while (n_iter > 0) {
-      bool ran_on_device = false;
-      const bool want_device = p->host_loop == 2;
-      if (want_device && g->ctx->device_loop) {
+      bool ran_on_device = swept;
+      swept = false;
+      if (!ran_on_device && p->host_loop == 0 && g->loop_plan) {
+        bool unsupported = false;
+        NIDO_TRY(persistent_sweeps(false, &unsupported));
+        ran_on_device = !unsupported;
+      } else if (!ran_on_device && p->host_loop == 2 && g->ctx->device_loop) {
         bool unsupported = false;
         NIDO_TRY(device_sweeps(&unsupported));
         if (unsupported) g->ctx->device_loop = false;
@@ -921,7 +966,7 @@ extern "C" int nido_batch_run(nido_batch B, const nido_params* p, int64_t* out_c
         listed_v = listed_e = 0;
         for (int32_t i : act)
           if (flags[i]) { it.push_back(i); listed_v += base[i + 1] - base[i]; listed_e += edges[i]; }
-        NIDO_TRY(batch_list(B, it, base, &ql, true));
+        NIDO_TRY(batch_list(B, it, base, listed_e, &ql, true));
         lap(2);
       }
     }

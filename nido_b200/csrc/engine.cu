@@ -226,7 +226,8 @@ extern "C" int nido_ctx_create(int device, size_t hbm_budget_bytes, nido_ctx* ou
   if (prop.major != 10)
     return nido_set_error(NIDO_E_NODEVICE, "device %d is sm_%d%d; this build targets sm_100a", device,
                           prop.major, prop.minor);
-  NIDO_TRY(nido::move_init_attributes());
+  NIDO_TRY(nido::move_init_attributes(false));
+  NIDO_TRY(nido::phase_loop_init(false));
   nido_ctx ctx = new (std::nothrow) nido_ctx_s();
   if (!ctx) return nido_set_error(NIDO_E_NOMEM, "host allocation failed");
   ctx->device = device;
@@ -1020,17 +1021,22 @@ extern "C" int nido_run(nido_graph g, const nido_params* p, int64_t* out_comm, n
     NIDO_TRY(nido::launch_singleton(g));
     double Q = 0., Q_old = 0.;
     int64_t loops = 0;
-    const bool want_device = p->host_loop == 2;
-    bool host_loop = !want_device || !g->ctx->device_loop || (p->verbose && p->max_iter > nido::kLoopLogCap);
-    if (!host_loop) {
-      // the phase's iteration loop as one device-resident CUDA graph
+    // the phase's iterations: on the persistent kernel where the phase is small
+    // (the default), as a device-resident CUDA graph (host_loop = 2), else
+    // driven from here
+    bool host_loop = true;
+    const bool want_log = p->verbose != 0;
+    if (p->host_loop != 1 && !(want_log && p->max_iter > nido::kLoopLogCap)) {
       nido::PhaseLoop r;
-      bool unsupported = false;
-      NIDO_TRY(nido::device_phase_loop(g, p->tie_mode, tau, p->max_iter, p->verbose != 0, &r, &unsupported));
-      if (unsupported) {
-        g->ctx->device_loop = false;  // this driver has no conditional graph nodes
-        host_loop = true;
-      } else {
+      bool unsupported = p->host_loop == 2 && !g->ctx->device_loop;
+      if (p->host_loop == 0) {
+        NIDO_TRY(nido::persistent_phase_loop(g, p->tie_mode, tau, p->max_iter, want_log, nullptr, &r, &unsupported));
+      } else if (!unsupported) {
+        NIDO_TRY(nido::device_phase_loop(g, p->tie_mode, tau, p->max_iter, want_log, &r, &unsupported));
+        if (unsupported) g->ctx->device_loop = false;  // this driver has no conditional graph nodes
+      }
+      if (!unsupported) {
+        host_loop = false;
         Q_old = r.q_old;
         Q = r.q;
         loops = r.loops;

@@ -210,6 +210,8 @@ struct nido_graph_s {
   std::vector<int64_t> cuts;     // host batch cuts (nbatches+1)
   std::vector<int64_t> tier_off; // host: nbatches*kNumTiers+1 offsets into perm
   bool bins_valid = false;
+  int64_t plan_ne = -1;          // many graphs: edges of the listed graphs (-1: ne)
+  bool loop_plan = false;        // the tier lists are cut for the persistent phase loop
   int64_t max_degree = 0;
   TierConfig cfg;
   bool tuned = false;
@@ -291,7 +293,7 @@ int launch_move(nido_graph_s* g, int batch, int tie, cudaEvent_t ev_start, cudaE
 int launch_move_tiers(nido_graph_s* g, int batch, int tie);  // enqueue only (capturable)
 int check_bounded_wait(nido_ctx_s* ctx, int32_t* gave_up, int32_t* waited_ms);  // move.cu
 int plan_hubs(nido_graph_s* g);          // per phase, after the tier lists
-int move_init_attributes();              // once per device
+int move_init_attributes(bool many);     // kernels of one graph / of many graphs
 // times `sweeps` move sweeps (no commit) for candidate tier configurations
 // and keeps the fastest in g->cfg (engine.cu); clobbers newc
 int tune_tiers(nido_graph_s* g, int tie, int sweeps, double* best_ms);
@@ -302,10 +304,37 @@ struct PhaseLoop {
   int64_t loops = 0;
   double move_ms = 0., q_ms = 0.;
   double build_ms = 0.;     // host time to capture and instantiate the loop graph
+  unsigned long long counters[4] = {0, 0, 0, 0};  // many graphs: iterating, restoring, their vertices
   std::vector<double> log;  // Qtmp, dQ of every iteration (with want_log)
 };
 int device_phase_loop(nido_graph_s* g, int tie, double tau, int64_t max_iter, bool want_log, PhaseLoop* r,
                       bool* unsupported);
+// the same as one persistent kernel (phase_loop.cu)
+// Phases of at most kLoopMaxEdges edges, or kLoopMaxBatchEdges a batch, run on it by
+// default.  A batch of a few hundred thousand edges is launch-bound on the
+// per-tier kernels: 22.8 M edges in 32 batches take 1.4 ms a sweep on them and
+// 0.95 ms here, 2.0 M edges in one batch 0.16 and 0.10 ms.  The per-tier
+// kernels keep more warps resident and win above: 57.9 M edges in 32 batches 3.0
+// against 3.3 ms, 7.6 M in two batches (reference tie rule) 0.5 against 0.7 ms.
+constexpr int64_t kLoopMaxEdges = (int64_t)4 << 20;
+constexpr int64_t kLoopMaxBatchEdges = (int64_t)1 << 20;
+bool loop_plan_fits(const nido_graph_s* g, int nb);  // the phase (nb batches) is one of those (phase.cu)
+struct LoopGraphs {  // many graphs: the listed graphs and their loop state (device)
+  const int32_t* gl;
+  const int64_t* qoff;
+  int nl, nbig;
+  double* modv;
+  double* q;
+  double* q_old;         // null: Q is valid already
+  int32_t* loops_phase;
+  int64_t* loops_total;
+  int32_t* giter;
+  int32_t* grest;
+  int64_t relist_below;  // leave the loop when the iterating graphs hold fewer vertices
+};
+int phase_loop_init(bool many);
+int persistent_phase_loop(nido_graph_s* g, int tie, double tau, int64_t max_iter, bool want_log, const LoopGraphs* many,
+                          PhaseLoop* r, bool* unsupported);
 // coarsening (coarsen.cu)
 int launch_aggregation(nido_graph_s* g, int* done);
 

@@ -640,24 +640,27 @@ int launch_tiers(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
 }
 }  // namespace
 
-int move_init_attributes() {
+// attributes of the kernels of one graph (contexts) or many (batches)
+int move_init_attributes(bool many) {
+  if (many) {
+    NIDO_TRY((init_mode<true, false>()));
+    return init_mode<true, true>();
+  }
   NIDO_TRY(cluster_init());
   NIDO_TRY((init_mode<false, false>()));
-  NIDO_TRY((init_mode<false, true>()));
-  NIDO_TRY((init_mode<true, false>()));
-  return init_mode<true, true>();
+  return init_mode<false, true>();
 }
 
-namespace {
 MoveArgs move_args(nido_graph_s* g) {
   double zh = 0., zl = 0.;
   if (!g->gid && g->int_weights) mass_reciprocal(g->m, &zh, &zl);
-  return MoveArgs{g->off, g->adj, g->w, g->comm, g->k, g->a, g->newc, g->m,
+  return MoveArgs{g->off, g->adj, g->w, g->k, g->comm, g->a, g->newc, g->m,
                   reinterpret_cast<unsigned long long*>(g->dcount + 1), g->gid, g->mg, zh, zl,
                   g->int_weights ? g->zg : nullptr,
                   g->int_weights ? 1 : 0, g->nv};
 }
 
+namespace {
 int tiers_direct(nido_graph_s* g, int batch, int tie, const MoveArgs& p) {
   if (g->gid) return p.ints ? launch_tiers<true, true>(g, batch, tie, p) : launch_tiers<true, false>(g, batch, tie, p);
   return p.ints ? launch_tiers<false, true>(g, batch, tie, p) : launch_tiers<false, false>(g, batch, tie, p);

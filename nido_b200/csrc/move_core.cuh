@@ -15,10 +15,11 @@ struct MoveArgs {
   const int64_t* __restrict__ off;
   const int32_t* __restrict__ adj;
   const double* __restrict__ w;
-  const int32_t* __restrict__ comm;
   const double* __restrict__ k;
-  const double* __restrict__ a;
-  int32_t* __restrict__ newc;
+  // not __restrict__: the persistent phase loop writes them between sweeps
+  const int32_t* comm;
+  const double* a;
+  int32_t* newc;
   double m;
   unsigned long long* err;  // probe-limit failures (never expected)
   // many-graph mode: graph of every vertex and mass of every graph (null for
@@ -36,6 +37,8 @@ struct MoveArgs {
   int ints;
   int64_t nv;  // vertices of the current graph (all graphs in many-graph mode)
 };
+
+MoveArgs move_args(nido_graph_s* g);  // of the current phase (move.cu)
 
 // The mass a vertex's gains are divided by, with its reciprocal zh = RN(1/m)
 // and zl = (1 - m zh) zh (zh = 0: use the divide).

@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "cuts.cuh"
 #include "engine.cuh"
+#include "phase_core.cuh"
 #include "primitives.cuh"
 
 namespace nido {
@@ -127,55 +128,15 @@ __global__ void k_comm_weights(int64_t nv, const int32_t* __restrict__ comm,
 // community, which takes the contention off communities many vertices join.
 // The atomics' order is not fixed (as in the reference); on integer weights
 // every sum is exact.
-__device__ __forceinline__ void warp_community_add(double* a, int c, double x, bool on) {
-  const int lane = threadIdx.x & 31;
-  const unsigned peers = __match_any_sync(NIDO_FULL_MASK, on ? c : -1);
-  double s = 0.;
-  unsigned rem = on ? peers : 0u;
-  const int maxcnt = __reduce_max_sync(NIDO_FULL_MASK, (unsigned)__popc(rem));
-  for (int it = 0; it < maxcnt; ++it) {
-    const int src = rem ? __ffs(rem) - 1 : lane;
-    const double y = __shfl_sync(NIDO_FULL_MASK, x, src);
-    if (rem) { s += y; rem &= rem - 1; }
-  }
-  if (on && lane == __ffs(peers) - 1) atomicAdd(&a[c], s);
-}
-
 __global__ void k_commit(int64_t v0, int64_t v1, const double* __restrict__ k,
                          int32_t* __restrict__ comm, int32_t* __restrict__ newc,
-                         double* __restrict__ a, int64_t* __restrict__ moved,
-                         const int32_t* __restrict__ gate) {
+                         double* __restrict__ a, const int32_t* __restrict__ gate) {
   if (gate && *gate == 0) return;  // the device-resident loop's restore, when not needed
-  int64_t cnt = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   // the loop runs warp-uniformly (the warp's first lane decides)
   for (int64_t base = v0 + blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); base < v1; base += stride) {
     const int64_t v = base + (threadIdx.x & 31);
-    int32_t src = 0, dst = 0;
-    double kv = 0.;
-    const bool in = v < v1;
-    if (in) {
-      src = comm[v];
-      dst = newc[v];
-    }
-    const bool mv = in && src != dst;
-    if (mv) {
-      kv = k[v];
-      ++cnt;
-    }
-    if (__any_sync(NIDO_FULL_MASK, mv)) {
-      warp_community_add(a, src, -kv, mv);
-      warp_community_add(a, dst, kv, mv);
-    }
-    if (in) {
-      comm[v] = dst;
-      newc[v] = src;
-    }
-  }
-  if (moved) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(NIDO_FULL_MASK, cnt, o);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd((unsigned long long*)moved, (unsigned long long)cnt);
+    commit_vertex(v, v < v1, k, comm, newc, a);
   }
 }
 
@@ -195,63 +156,16 @@ __global__ void k_commit_spans(PermSpans r, const int32_t* __restrict__ perm, co
     const int64_t x = base + (threadIdx.x & 31);
     const bool in = x < total;
     int v = 0;
-    int32_t src = 0, dst = 0;
-    double kv = 0.;
     if (in) {
       int t = 0;
       while (r.pre[t + 1] <= x) ++t;
       v = perm[r.start[t] + (x - r.pre[t])];
-      src = comm[v];
-      dst = newc[v];
     }
-    const bool mv = in && src != dst;
-    if (mv) kv = k[v];
-    if (__any_sync(NIDO_FULL_MASK, mv)) {
-      warp_community_add(a, src, -kv, mv);
-      warp_community_add(a, dst, kv, mv);
-    }
-    if (in) {
-      comm[v] = dst;
-      newc[v] = src;
-    }
+    commit_vertex(v, in, k, comm, newc, a);
   }
 }
 
 // ---- modularity -------------------------------------------------------------------
-// Sum of w[j] over j = j0, j0+step, ... < e with comm[adj[j]] == own, added in
-// that order; four edges' loads (bounds-guarded) are issued before any is
-// added, so four dependent gathers are in flight per lane at every degree.
-__device__ __forceinline__ double own_weight(const int32_t* __restrict__ adj, const double* __restrict__ w,
-                                             const int32_t* __restrict__ comm, int32_t own, int64_t j0,
-                                             int64_t e, int step) {
-  double x = 0.;
-  for (int64_t j = j0; j < e; j += 4 * (int64_t)step) {
-    int u[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int64_t jk = j + k * (int64_t)step;
-      u[k] = jk < e ? adj[jk] : -1;
-    }
-    int c[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) c[k] = u[k] >= 0 ? comm[u[k]] : 0;
-    // only in-community edges load their weight: a warp's 32-byte weight
-    // sectors with no such edge are never fetched (most of them while the
-    // communities are small); the sum and its order are unchanged
-    bool in[4];
-    double wt[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      in[k] = u[k] >= 0 && c[k] == own;
-      wt[k] = in[k] ? w[j + k * (int64_t)step] : 0.;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (in[k]) x += wt[k];
-  }
-  return x;
-}
-
 // Stage 1: per-vertex in-community weight (self-loops included), one group of
 // G lanes per vertex; lane l sums edges l, l+G, ... then a fixed tree.
 template <int G>
@@ -259,22 +173,9 @@ __global__ void k_q_self_group(const int32_t* __restrict__ list, int64_t n,
                                const int64_t* __restrict__ off, const int32_t* __restrict__ adj,
                                const double* __restrict__ w, const int32_t* __restrict__ comm,
                                double* __restrict__ selfv) {
-  constexpr int VPW = 32 / G;
-  const int lane = threadIdx.x & 31, gl = lane & (G - 1), gid = lane / G;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t b = warp * VPW; b < n; b += nw * VPW) {
-    const int64_t idx = b + gid;
-    double x = 0.;
-    int v = 0;
-    if (idx < n) {
-      v = list[idx];
-      x = own_weight(adj, w, comm, comm[v], off[v] + gl, off[v + 1], G);
-    }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) x += __shfl_down_sync(NIDO_FULL_MASK, x, o, G);
-    if (gl == 0 && idx < n) selfv[v] = x;
-  }
+  q_self_list<G>(list, n, warp, nw, off, adj, w, comm, selfv);
 }
 
 template <int T>
@@ -287,17 +188,8 @@ __global__ void __launch_bounds__(T) k_q_self_cta(const int32_t* __restrict__ li
   __shared__ double ws[T / 32];
   for (int64_t idx = blockIdx.x; idx < n; idx += gridDim.x) {
     const int v = list[idx];
-    double x = own_weight(adj, w, comm, comm[v], off[v] + threadIdx.x, off[v + 1], T);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(NIDO_FULL_MASK, x, o);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.;
-      for (int i = 0; i < T / 32; ++i) s += ws[i];
-      selfv[v] = s;
-    }
-    __syncthreads();
+    const double s = q_self_block<T>(adj, w, comm, comm[v], off[v], off[v + 1], ws);
+    if (threadIdx.x == 0) selfv[v] = s;
   }
 }
 
@@ -318,17 +210,8 @@ __global__ void __launch_bounds__(256) k_q_self_seg(const int2* __restrict__ ite
     const int v = hub_v[it.x];
     const int64_t e0 = off[v] + (int64_t)it.y * kHubSeg;
     const int64_t e1 = min(off[v + 1], e0 + kHubSeg);
-    double x = own_weight(adj, w, comm, comm[v], e0 + threadIdx.x, e1, 256);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(NIDO_FULL_MASK, x, o);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.;
-      for (int i = 0; i < 8; ++i) s += ws[i];
-      part[idx] = s;
-    }
-    __syncthreads();
+    const double s = q_self_block<256>(adj, w, comm, comm[v], e0, e1, ws);
+    if (threadIdx.x == 0) part[idx] = s;
   }
 }
 
@@ -368,10 +251,7 @@ __global__ void k_q_groups(int64_t nv, int64_t S, int64_t ngroups, const double*
     ac += __shfl_down_sync(NIDO_FULL_MASK, ac, o, 16);
   }
   if ((t & 15) == 0 && g < ngroups) {
-    const double m = dm[0];
-    double x = __ddiv_rn(s, __dmul_rn(2., m));
-    x = __dsub_rn(x, __ddiv_rn(ac, __dmul_rn(__dmul_rn(4., m), m)));
-    modv[g] = __dadd_rn(0., x);
+    modv[g] = q_part(s, ac, dm[0]);
   }
 }
 
@@ -528,7 +408,7 @@ int launch_set_comm(nido_graph_s* g) {
 int launch_commit(nido_graph_s* g, int64_t v0, int64_t v1) {
   if (v1 <= v0) return NIDO_OK;
   k_commit<<<grid_for(v1 - v0, kThreads), kThreads, 0, g->ctx->stream>>>(v0, v1, g->k, g->comm,
-                                                                         g->newc, g->a, nullptr, nullptr);
+                                                                         g->newc, g->a, nullptr);
   NIDO_LAUNCH_CHECK();
   return NIDO_OK;
 }
@@ -557,7 +437,7 @@ int launch_commit_batch(nido_graph_s* g, int b) {
 int launch_commit_gated(nido_graph_s* g, int64_t v0, int64_t v1, const int32_t* gate) {
   if (v1 <= v0) return NIDO_OK;
   k_commit<<<grid_for(v1 - v0, kThreads), kThreads, 0, g->ctx->stream>>>(v0, v1, g->k, g->comm,
-                                                                         g->newc, g->a, nullptr, gate);
+                                                                         g->newc, g->a, gate);
   NIDO_LAUNCH_CHECK();
   return NIDO_OK;
 }
@@ -695,6 +575,17 @@ int launch_modularity_dev(nido_graph_s* g) {
   return NIDO_OK;
 }
 
+// Small phases run on the persistent phase loop; tier settings of the
+// caller's stay as they are.
+bool loop_plan_fits(const nido_graph_s* g, int nb) {
+  const TierConfig d;
+  const int64_t ne = g->gid && g->plan_ne >= 0 ? g->plan_ne : g->ne;
+  return !g->host_edges && (ne <= kLoopMaxEdges || ne / nb <= kLoopMaxBatchEdges) && g->cfg.warp_max == d.warp_max &&
+         g->cfg.ctas_max == d.ctas_max && g->cfg.ctam_max == d.ctam_max && g->cfg.ctal_max == d.ctal_max &&
+         g->cfg.ctax_max == d.ctax_max && !g->cfg.hub_clusters && !g->cfg.staged_edges &&
+         g->cfg.hub_wave_slots == d.hub_wave_slots;
+}
+
 int build_batches(nido_graph_s* g) {
   cudaStream_t s = g->ctx->stream;
   const bool multi = g->gid != nullptr;  // many graphs: per-graph cuts in g->gcuts
@@ -733,13 +624,16 @@ int build_batches(nido_graph_s* g) {
   }
   NIDO_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int64_t) * (nkeys + 1), s));
   NIDO_CUDA_TRY(cudaMemsetAsync(maxdeg, 0, sizeof(unsigned long long), s));
+  // the persistent phase loop's CTA tiers end at its table's 3072 edges, larger
+  // vertices are hubs
+  g->loop_plan = loop_plan_fits(g, nb);
+  const int ctal = g->loop_plan ? kCtaLMaxDeg : g->cfg.ctal_max, ctax = g->loop_plan ? kCtaLMaxDeg : g->cfg.ctax_max;
   if (nv > 0) {
     k_tier_keys<<<grid_for(nv, kThreads), kThreads, 0, s>>>(g->off, nv, dcuts, nb, keys, (uint32_t*)g->perm,
                                                            counts, maxdeg, g->gid, g->gbase, g->gcuts,
                                                            g->gactive, g->vbatch, colored ? g->vcolor : nullptr,
                                                            TierThresholds{g->cfg.warp_max, g->cfg.ctas_max,
-                                                                          g->cfg.ctam_max, g->cfg.ctal_max,
-                                                                          g->cfg.ctax_max});
+                                                                          g->cfg.ctam_max, ctal, ctax});
     NIDO_LAUNCH_CHECK();
     int bits = 0;
     while (((int64_t)1 << bits) < nkeys + 1) ++bits;
