@@ -191,6 +191,9 @@ __global__ void k_set_ids(const int64_t* __restrict__ c64, int64_t nv, int32_t* 
 constexpr unsigned kGrid = 148 * 8;
 
 int prepare_phase(nido_graph g) {
+  bool staged = false;
+  NIDO_TRY(nido::phase_setup(g, &staged));
+  if (!staged) return NIDO_OK;
   NIDO_TRY(nido::launch_vertex_weights(g));
   NIDO_TRY(nido::launch_mass(g));
   g->bins_valid = false;
@@ -228,6 +231,7 @@ extern "C" int nido_ctx_create(int device, size_t hbm_budget_bytes, nido_ctx* ou
                           prop.major, prop.minor);
   NIDO_TRY(nido::move_init_attributes(false));
   NIDO_TRY(nido::phase_loop_init(false));
+  NIDO_TRY(nido::phase_step_init());
   nido_ctx ctx = new (std::nothrow) nido_ctx_s();
   if (!ctx) return nido_set_error(NIDO_E_NOMEM, "host allocation failed");
   ctx->device = device;
@@ -1106,11 +1110,14 @@ extern "C" int nido_run(nido_graph g, const nido_params* p, int64_t* out_comm, n
       int d = 0;
       lap(1);
       NIDO_TRY(at.begin(s));
-      NIDO_TRY(nido::launch_aggregation(g, &d));
+      bool staged = p->host_loop != 0;  // the separate stages
+      if (!staged) NIDO_TRY(nido::phase_step(g, &d, &staged));
+      const bool set_up = !staged;
+      if (staged) NIDO_TRY(nido::launch_aggregation(g, &d));
       NIDO_TRY(at.end(s));
       lap(3);
       done = d != 0;
-      if (!done) NIDO_TRY(prepare_phase(g));
+      if (!done && !set_up) NIDO_TRY(prepare_phase(g));
       lap(4);
     } else {
       done = true;

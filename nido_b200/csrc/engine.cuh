@@ -335,6 +335,12 @@ struct LoopGraphs {  // many graphs: the listed graphs and their loop state (dev
 int phase_loop_init(bool many);
 int persistent_phase_loop(nido_graph_s* g, int tie, double tau, int64_t max_iter, bool want_log, const LoopGraphs* many,
                           PhaseLoop* r, bool* unsupported);
+// A small phase's coarsening with the next phase's set-up (k, m, cuts, tier
+// lists), or the set-up alone, as one kernel (phase_step.cu).
+// *unsupported: nothing was done, the separate stages are to run.
+int phase_step_init();
+int phase_step(nido_graph_s* g, int* done, bool* unsupported);
+int phase_setup(nido_graph_s* g, bool* unsupported);
 // coarsening (coarsen.cu)
 int launch_aggregation(nido_graph_s* g, int* done);
 

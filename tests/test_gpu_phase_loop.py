@@ -1,8 +1,10 @@
-"""The persistent phase loop (the default for small phases) against the host
-driven loop (host_loop): the same stages in one kernel, so on weights whose
-sums are exact every partition, every phase's Q and every loop count are
-identical, under both tie rules, for integer and FP64 tables, with hubs of one
-and of several segments, colour-class batches, loop caps and undone sweeps."""
+"""The persistent kernels of small phases (the phase loop, and the coarsening with
+the next phase's set-up; the default) against the host driven loop and the
+separate stages (host_loop): on weights whose sums are exact every partition,
+every phase's Q and every loop count are identical, under both tie rules, for
+integer and FP64 tables, with hubs of one and of several segments, communities of
+more and of fewer members than a block lists in order, colour-class batches,
+loop caps and undone sweeps."""
 import numpy as np
 import pytest
 
@@ -39,6 +41,7 @@ def same(a, b):
     assert sa.phases == n and sa.total_loops == sb.total_loops
     assert np.array_equal(bits(sa.q_phase[:n]), bits(sb.q_phase[:n]))
     assert list(sa.loops_phase[:n]) == list(sb.loops_phase[:n])
+    assert list(sa.nv_phase[:n]) == list(sb.nv_phase[:n]) and list(sa.ne_phase[:n]) == list(sb.ne_phase[:n])
     assert sa.move_bytes == sb.move_bytes and sa.edges_scanned == sb.edges_scanned
 
 
