@@ -14,7 +14,11 @@
 // place in the coarse CSR in the reference's first-occurrence order.  Equal
 // neighbours of a 32-edge chunk are folded in edge order before they are
 // added; across chunks the adds are atomic (exact for integer weights, as in
-// the CTA tiers of coarsen.cu).
+// the CTA tiers of coarsen.cu).  In FP64 phases the weights of coarse vertices
+// of at most 1024 member edges are added in list order instead: every edge notes
+// its entry and weight at its list position, and a warp walks the list.  Up to
+// 256 each weight is added to its entry, as in the warp tier of coarsen.cu, above
+// each 32-edge chunk's sum, as in its CTA tiers (in some order there).
 #include <string.h>
 
 #include <algorithm>
@@ -83,6 +87,7 @@ struct StepArgs {
   PhaseCtl* ctl;
   unsigned long long* err;
   bool coarsen;             // false: only the set-up of the current graph
+  bool ordered;             // FP64 phase: short lists are summed in list order
   int warp, ctas, ctam, ctal;
 };
 
@@ -164,20 +169,46 @@ __device__ __forceinline__ void scan_apply(int64_t n, Get get, const int32_t* bs
   if (blockIdx.x == 0 && threadIdx.x == 0) put(n, all);
 }
 
-__device__ __forceinline__ void table_put(const StepArgs& A, int cu, int cv, double x, unsigned at) {
+// member edges of a list summed in order: a chunk takes a warp about two
+// microseconds (planted, 7,900 edges a list: 2.7 ms a run in order, 2.1 without)
+constexpr int kStepOrdered = 1024;
+constexpr int kStepOneByOne = 256;   // and of one whose weights are added one by one
+
+// Entry of (cu, cv) with `at` among its positions; adds x unless the list is
+// summed in order.
+__device__ __forceinline__ int table_put(const StepArgs& A, int cu, int cv, bool add, double x, unsigned at) {
   const unsigned long long key = (unsigned long long)(unsigned)cu << 32 | (unsigned)cv;
   unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> 32) & A.mask;
   for (unsigned probe = 0; probe <= A.mask; ++probe) {
     unsigned long long o = __ldcg(A.keys + h);
     if (o == kNoEntry) o = atomicCAS(A.keys + h, kNoEntry, key);
     if (o == kNoEntry || o == key) {
-      atomicAdd(A.vals + h, x);
+      if (add) atomicAdd(A.vals + h, x);
       if (__ldcg(A.first + h) > at) atomicMin(A.first + h, at);
-      return;
+      return (int)h;
     }
     h = (h + probe + 1) & A.mask;
   }
   atomicAdd(A.err, 1ull);
+  return 0;
+}
+
+// One edge a lane (ok): list position `at`, from coarse vertex cu to cv with
+// weight x; peers: the lanes with the same entry.
+__device__ __forceinline__ void put_chunk(const StepArgs& A, unsigned peers, bool ok, int cu, int cv, double x,
+                                          unsigned at) {
+  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+  const bool in_order = A.ordered && ok && A.deg[cu] <= kStepOrdered;
+  const double s = fold_peers(peers, ok, x);
+  int h = 0;
+  if (ok && lane == leader) h = table_put(A, cu, cv, !in_order, s, at);
+  if (A.ordered) {
+    h = __shfl_sync(NIDO_FULL_MASK, h, leader);
+    if (in_order) {  // the coarse graph's arrays are free until the entries are written
+      A.cadj[at] = h;
+      A.cw[at] = x;
+    }
+  }
 }
 
 // Edges [j0, j1) of vertex v, 32 at a time every `stride`, by a warp.
@@ -193,9 +224,7 @@ __device__ __forceinline__ void put_edges(const StepArgs& A, int v, int64_t e0, 
       cv = A.newid[A.adj[e0 + j]];
       x = A.w[e0 + j];
     }
-    const unsigned peers = __match_any_sync(NIDO_FULL_MASK, cv);
-    const double s = fold_peers(peers, ok, x);
-    if (ok && lane == __ffs(peers) - 1) table_put(A, cu, cv, s, (unsigned)at + (unsigned)j);
+    put_chunk(A, __match_any_sync(NIDO_FULL_MASK, cv), ok, cu, cv, x, (unsigned)at + (unsigned)j);
   }
 }
 
@@ -205,23 +234,59 @@ __device__ __forceinline__ void put_groups(const StepArgs& A, const int32_t* lis
   const int lane = threadIdx.x & 31, gl = lane & (G - 1), gid = lane / G;
   for (int64_t b = gw * (32 / G); b < n; b += nw * (32 / G)) {
     const int64_t i = b + gid;
-    int v = 0, cu = 0, cv = -1;
+    int cu = 0, cv = -1;
+    unsigned at = 0;
     double x = 0.;
     bool ok = false;
     if (i < n) {
-      v = list[i];
+      const int v = list[i];
       const int64_t e0 = A.off[v];
       ok = gl < A.off[v + 1] - e0;
       cu = A.newid[v];
+      at = (unsigned)A.pos[v] + (unsigned)gl;
       if (ok) {
         cv = A.newid[A.adj[e0 + gl]];
         x = A.w[e0 + gl];
       }
     }
-    const unsigned peers =
-        __match_any_sync(NIDO_FULL_MASK, ((unsigned long long)(unsigned)gid << 32) | (unsigned)cv);
-    const double s = fold_peers(peers, ok, x);
-    if (ok && lane == __ffs(peers) - 1) table_put(A, cu, cv, s, (unsigned)A.pos[v] + (unsigned)gl);
+    put_chunk(A, __match_any_sync(NIDO_FULL_MASK, ((unsigned long long)(unsigned)gid << 32) | (unsigned)cv), ok, cu, cv,
+              x, at);
+  }
+}
+
+// The lists summed in order, a warp per coarse vertex: the lanes' weights are
+// folded in lane (= list) order.
+__device__ __forceinline__ void sum_in_order(const StepArgs& A, int64_t nvp, int64_t gw, int64_t nw) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t c = gw; c < nvp; c += nw) {
+    const int D = A.deg[c], p = A.p0[c];
+    if (D > kStepOrdered) continue;
+    // the next chunk's entries and weights are loaded ahead
+    int hn = lane < D ? A.cadj[p + lane] : -1;
+    double xn = lane < D ? A.cw[p + lane] : 0.;
+    for (int b = 0; b < D; b += 32) {
+      const bool ok = b + lane < D;
+      const int h = hn;
+      const double x = xn;
+      hn = -1;
+      if (b + 32 + lane < D) {
+        hn = A.cadj[p + b + 32 + lane];
+        xn = A.cw[p + b + 32 + lane];
+      }
+      const unsigned peers = __match_any_sync(NIDO_FULL_MASK, h);
+      const bool leads = ok && lane == __ffs(peers) - 1;
+      const double old = leads ? A.vals[h] : 0.;
+      double acc = D <= kStepOneByOne ? old : 0.;
+      unsigned rem = ok ? peers : 0u;
+      const int maxcnt = __reduce_max_sync(NIDO_FULL_MASK, (unsigned)__popc(rem));
+      for (int i = 0; i < maxcnt; ++i) {
+        const int src = rem ? __ffs(rem) - 1 : lane;
+        const double y = __shfl_sync(NIDO_FULL_MASK, x, src);
+        if (rem) { acc += y; rem &= rem - 1; }
+      }
+      if (leads) A.vals[h] = D <= kStepOneByOne ? acc : old + acc;
+      __syncwarp();
+    }
   }
 }
 
@@ -381,6 +446,7 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
       const unsigned f = __ldcg(A.first + i);
       atomicOr(A.bm + (f >> 5), 1u << (f & 31));
     }
+    if (A.ordered) sum_in_order(A, nvp, gw, nw);
     STEP_BARRIER();
     auto bits = [&](int64_t i) { return __popc(__ldcg(A.bm + i)); };
     scan_sums(A.nwords, bits, A.bsum, ws);
@@ -562,6 +628,7 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
   A.toff = A.cuts + nb + 1;
   A.tier_off = tier;
   A.coarsen = coarsen;
+  A.ordered = !g->int_weights;
   if (coarsen) {
     int64_t slots = 64;
     while (slots < 2 * ne) slots <<= 1;
