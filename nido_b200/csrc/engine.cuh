@@ -72,6 +72,10 @@ struct nido_ctx_s {
   size_t used = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<cudaEvent_t> move_ev;  // 2 per batch, for per-iteration move timing
+  // events of a run (start, end, two sections' timers) and of an upload, made
+  // once: creating and destroying them in every run took the serving loop's
+  // workers milliseconds, waiting for one another in the driver
+  cudaEvent_t run_ev[10] = {}, upload_ev[16] = {};
   // side streams of the move sweep: the degree tiers of one batch touch
   // disjoint vertices, so the hub chain and the CTA tiers run beside the
   // small-degree tiers (fork and join events on the context's stream)
