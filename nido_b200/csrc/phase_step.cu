@@ -56,7 +56,8 @@ struct StepArgs {
   int32_t* clus;
   int32_t* perm;
   const int64_t* tier_off;  // of the finished phase, kNumTiers * nb + 1
-  int nb;
+  int nb;                   // its batches
+  int nbn;                  // batches of the next phase; 0: no cuts and lists (colour classes)
   const int2* items;        // its hub segments
   int64_t nitems;
   const int32_t* hub_v;
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
   }
   // ---- set-up of the next phase: k (lane l sums edges l, l+32, ... then a
   // shuffle-down tree, graph_cuda.cu:302-346), weight flags, cuts
-  const int nb = A.nb;
+  const int nb = A.nbn;
   const int nkeys = kNumTiers * nb;
   {
     unsigned long long bad = 0;
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
       if (amax > 0. && __ldcg(&A.out->flags[1]) < ab) atomicMax(&A.out->flags[1], ab);
     }
     for (int64_t i = gt; i < 2 * (nkeys + 1); i += nt) A.counts[i] = 0;  // and the cursors behind them
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kStepThreads - 1) batch_cuts(noff, nvn, nb, A.cuts, A.parts);
+    if (nb > 0 && blockIdx.x == gridDim.x - 1 && threadIdx.x == kStepThreads - 1) batch_cuts(noff, nvn, nb, A.cuts, A.parts);
   }
   STEP_BARRIER();
   // ---- mass partials (graph_cuda.cu:1786-1804), tier and batch of every vertex
@@ -518,7 +519,7 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(NIDO_FULL_MASK, x, o);
     if (lane == 0) A.part[b] = x;
   }
-  {
+  if (nb > 0) {
     unsigned md = 0;
     for (int64_t base = gt - lane; base < nvn; base += nt) {
       const int64_t v = base + lane;
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
   }
   STEP_BARRIER();
   // ---- list offsets (every block for itself), the lists, and m
-  {
+  if (nb > 0) {
     int run = 0;
     for (int t = 0; t <= nkeys; t += kStepThreads) {
       const int i = t + (int)threadIdx.x;
@@ -566,10 +567,10 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
       at = __shfl_sync(NIDO_FULL_MASK, at, leader);
       if (key >= 0) A.perm[soff[key] + at + __popc(peers & lanemask_lt())] = (int32_t)v;
     }
-    if (blockIdx.x == gridDim.x - 1) {
-      const double s = loop_reduce_1024(A.part, 4096, wd);
-      if (threadIdx.x == 0) A.out->m = 0.5 * s;
-    }
+  }
+  if (blockIdx.x == gridDim.x - 1) {
+    const double s = loop_reduce_1024(A.part, 4096, wd);
+    if (threadIdx.x == 0) A.out->m = 0.5 * s;
   }
 #undef STEP_BARRIER
 }
@@ -578,12 +579,14 @@ int64_t g_step_resident = kSMs;
 
 int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
   cudaStream_t s = g->ctx->stream;
-  const int nb = g->nb_user;
+  const bool colored = g->color_mode;  // the coarse graph is coloured first: no lists here
+  const int nb = colored ? 0 : g->nb_user;
   const int nkeys = kNumTiers * nb;
+  const int64_t nold = (int64_t)kNumTiers * g->nbatches;
   *unsupported = true;
   const int64_t nv = g->nv, ne = g->ne;
-  if (nv < 1 || nv > kStepMaxEdges || ne > kStepMaxEdges || nkeys > kStepKeys || g->gid || g->color_mode ||
-      g->host_edges || !loop_plan_fits(g, nb) || (coarsen && (!g->loop_plan || !g->bins_valid || g->nbatches != nb)))
+  if (nv < 1 || nv > kStepMaxEdges || ne > kStepMaxEdges || nkeys > kStepKeys || g->gid || g->host_edges ||
+      !loop_plan_fits(g, std::max(nb, 1)) || (coarsen && (!g->loop_plan || !g->bins_valid)))
     return NIDO_OK;
   StepArgs A;
   memset(&A, 0, sizeof(A));
@@ -596,7 +599,8 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
   A.k = g->k;
   A.clus = g->clus;
   A.perm = g->perm;
-  A.nb = nb;
+  A.nb = g->nbatches;
+  A.nbn = nb;
   A.nitems = g->nhubs > 0 ? g->hub_nitems : 0;
   A.items = g->hub_items;
   A.hub_v = g->hub_v;
@@ -606,7 +610,7 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
   const int64_t nres = (int64_t)sizeof(StepOut) / 8 + (nb + 1) + (nkeys + 1);
   int64_t* res = ar.take<int64_t>(nres);
   A.ctl = ar.take<PhaseCtl>(1);
-  int64_t* tier = ar.take<int64_t>(nkeys + 1);
+  int64_t* tier = ar.take<int64_t>(nold + 1);
   A.parts = ar.take<int64_t>(nb + 2);
   A.counts = ar.take<int32_t>(2 * (nkeys + 1));
   A.bsum = ar.take<int32_t>(2 * blocks);
@@ -653,7 +657,7 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
     A.coff = g->off2;
     A.cadj = g->adj2;
     A.cw = g->w2;
-    NIDO_CUDA_TRY(cudaMemcpyAsync(tier, g->tier_off.data(), sizeof(int64_t) * (nkeys + 1), cudaMemcpyHostToDevice, s));
+    NIDO_CUDA_TRY(cudaMemcpyAsync(tier, g->tier_off.data(), sizeof(int64_t) * (nold + 1), cudaMemcpyHostToDevice, s));
   }
   A.err = reinterpret_cast<unsigned long long*>(g->dcount + 1);
   A.warp = g->cfg.warp_max;
@@ -694,13 +698,17 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
   // where the separate stages look for them
   NIDO_CUDA_TRY(cudaMemcpyAsync(g->dm, &A.out->m, sizeof(double), cudaMemcpyDeviceToDevice, s));
   NIDO_CUDA_TRY(cudaMemcpyAsync(g->dcount + 2, A.out->flags, sizeof(A.out->flags), cudaMemcpyDeviceToDevice, s));
+  double amax = 0.;
+  memcpy(&amax, &o.flags[1], sizeof(amax));
+  g->int_weights = o.flags[0] == 0 && amax < 2147483648.0;
+  if (colored) {
+    g->bins_valid = false;
+    return build_batches(g);
+  }
   g->nbatches = nb;
   const int64_t* cuts = h.data() + sizeof(StepOut) / 8;
   g->cuts.assign(cuts, cuts + nb + 1);
   g->tier_off.assign(cuts + nb + 1, cuts + nb + 1 + nkeys + 1);
-  double amax = 0.;
-  memcpy(&amax, &o.flags[1], sizeof(amax));
-  g->int_weights = o.flags[0] == 0 && amax < 2147483648.0;
   g->max_degree = (int64_t)o.maxdeg;
   g->loop_plan = true;
   g->bins_valid = true;
