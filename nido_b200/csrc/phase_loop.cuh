@@ -223,7 +223,12 @@ __global__ void __launch_bounds__(kLoopThreads, 4) k_phase_loop(const __grid_con
           }
           rot = n % gridDim.x;
         }
-        for (int tier = kTierCtaL; tier >= kTierCtaS; --tier) {
+        // A vertex of 100 to 190 edges takes a warp eight to ten microseconds,
+        // chunk after chunk, and a CTA three: while the batch has at most two of
+        // them a block, CTAs take the warp tier as well.
+        const int64_t nwarp = to[(int64_t)kTierWarp * nb + 1] - to[(int64_t)kTierWarp * nb];
+        const int lowest = nwarp <= 2 * (int64_t)gridDim.x ? kTierWarp : kTierCtaS;
+        for (int tier = kTierCtaL; tier >= lowest; --tier) {
           const int64_t l0 = to[(int64_t)tier * nb], n = to[(int64_t)tier * nb + 1] - l0;
           int64_t i = (int64_t)blockIdx.x - rot;
           if (i < 0) i += gridDim.x;
@@ -240,7 +245,7 @@ __global__ void __launch_bounds__(kLoopThreads, 4) k_phase_loop(const __grid_con
         int64_t wr = gw - rot * (kLoopThreads / 32);
         if (wr < 0) wr += nw;
         const int32_t* list = A.perm + to[(int64_t)kTierWarp * nb];
-        int64_t n = to[(int64_t)kTierWarp * nb + 1] - to[(int64_t)kTierWarp * nb];
+        int64_t n = lowest == kTierWarp ? 0 : nwarp;
         warp_list<kLoopWarpCap, kLoopWarpChunks, kMulti, kInts, kTie>(list, n, wr, nw, p, tw);
         auto rotate = [&](int64_t used) {
           wr -= used % nw;
