@@ -999,7 +999,9 @@ extern "C" int nido_batch_run(nido_batch B, const nido_params* p, int64_t* out_c
     NIDO_LAUNCH_CHECK();
     int done = 0;
     NIDO_CUDA_TRY(cudaEventRecord(re.a0, s));
-    NIDO_TRY(launch_aggregation(g, &done));
+    bool staged = p->host_loop != 0;  // the separate stages
+    if (!staged) NIDO_TRY(phase_step(g, &done, &staged));
+    if (staged) NIDO_TRY(launch_aggregation(g, &done));
     NIDO_CUDA_TRY(cudaEventRecord(re.a1, s));
     std::swap(g->gbase, g->gbase2);  // the clustering is in the new numbering either way
     k_post_agg<<<grid_for(np, 128), 128, 0, s>>>(B->plist, np, g->gbase2, g->gbase, B->gagg, B->gfin);

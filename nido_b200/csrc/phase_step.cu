@@ -87,7 +87,14 @@ struct StepArgs {
   StepOut* out;
   PhaseCtl* ctl;
   unsigned long long* err;
+  // many graphs: each one's first vertex, and its first coarse vertex (written).
+  // Vertices with a negative community are dropped; every vertex's edges are
+  // walked, as the lists hold only the graphs that still iterate.
+  const int64_t* gbase;
+  int64_t* gbase2;
+  int ng;
   bool coarsen;             // false: only the set-up of the current graph
+  bool setup;               // false: only the coarsening
   bool ordered;             // FP64 phase: short lists are summed in list order
   int warp, ctas, ctam, ctal;
 };
@@ -338,27 +345,38 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
     }
     for (int64_t i = gt; i < A.nwords; i += nt) A.bm[i] = 0u;
     STEP_BARRIER();
-    for (int64_t v = gt; v < nv; v += nt) A.used[A.comm[v]] = 1;
+    for (int64_t v = gt; v < nv; v += nt) {
+      const int c = A.comm[v];
+      if (c >= 0) A.used[c] = 1;
+    }
     STEP_BARRIER();
     auto used = [&](int64_t i) { return A.used[i]; };
     scan_sums(nv, used, A.bsum, ws);
     STEP_BARRIER();
     // the prefix replaces the flag of ids in use
     scan_apply(nv, used, A.bsum, [&](int64_t i, int x) {
-      if (i < nv) A.mo[i] = x;
-      else A.out->nvp = x;
+      A.mo[i] = x;
+      if (i == nv) A.out->nvp = x;
     }, ws);
     STEP_BARRIER();
     const int64_t nvp = (int64_t)__ldcg(&A.out->nvp);
     // ---- new ids, members and member edges of every coarse vertex; the
     // clustering of the original vertices is composed with the renumber
     for (int64_t v = gt; v < nv; v += nt) {
-      const int c = A.mo[A.comm[v]];
+      const int oc = A.comm[v], c = oc >= 0 ? A.mo[oc] : -1;
       A.newid[v] = c;
+      if (c < 0) continue;
       atomicAdd(A.cnt + c, 1);
       atomicAdd(A.deg + c, (int)(A.off[v + 1] - A.off[v]));
     }
-    for (int64_t i = gt; i < A.nv0; i += nt) A.clus[i] = A.mo[A.comm[A.clus[i]]];
+    for (int64_t i = gt; i < A.nv0; i += nt) {
+      const int v = A.clus[i];
+      if (v < 0) continue;
+      const int oc = A.comm[v];
+      A.clus[i] = oc >= 0 ? A.mo[oc] : -1;
+    }
+    if (A.gbase)  // communities never span graphs, so neither does the renumber
+      for (int64_t i = gt; i <= A.ng; i += nt) A.gbase2[i] = A.mo[A.gbase[i]];
     if (nvp == nv || nvp == 1) {  // graph_gpu.cpp:1391-1392
       if (lead) A.out->done = 1;
       return;
@@ -374,12 +392,15 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
     STEP_BARRIER();
     for (int64_t v = gt; v < nv; v += nt) {
       const int c = A.newid[v];
+      if (c < 0) continue;
       A.member[A.mo[c] + atomicAdd(A.cursor + c, 1)] = (int)v;
     }
     STEP_BARRIER();
     // ---- list position of every member's first edge
     for (int64_t v = gt; v < nv; v += nt) {
-      const int c = A.newid[v], m0 = A.mo[c], m1 = A.mo[c + 1];
+      const int c = A.newid[v];
+      if (c < 0) continue;
+      const int m0 = A.mo[c], m1 = A.mo[c + 1];
       if (m1 - m0 > kStepBigList) continue;
       int x = A.p0[c];
       for (int i = m0; i < m1; ++i) {
@@ -415,7 +436,10 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
     }
     STEP_BARRIER();
     // ---- edges into the table, by the finished phase's tier lists
-    {
+    if (A.gbase) {
+      for (int64_t v = gw; v < nv; v += nw)
+        if (A.newid[v] >= 0) put_edges(A, (int)v, A.off[v], 0, A.off[v + 1] - A.off[v], 32);
+    } else {
       const int64_t* to = A.tier_off;
       const int nb = A.nb;
       for (int64_t i = blockIdx.x; i < A.nitems; i += gridDim.x) {
@@ -474,6 +498,7 @@ __global__ void __launch_bounds__(kStepThreads, 4) k_phase_step(const __grid_con
     nvn = nvp;
     noff = A.coff;
     nwt = A.cw;
+    if (!A.setup) return;
   }
   // ---- set-up of the next phase: k (lane l sums edges l, l+32, ... then a
   // shuffle-down tree, graph_cuda.cu:302-346), weight flags, cuts
@@ -579,14 +604,17 @@ int64_t g_step_resident = kSMs;
 
 int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
   cudaStream_t s = g->ctx->stream;
-  const bool colored = g->color_mode;  // the coarse graph is coloured first: no lists here
-  const int nb = colored ? 0 : g->nb_user;
+  const bool colored = g->color_mode && !g->gid;  // the coarse graph is coloured first: no lists here
+  const bool many = g->gid != nullptr;            // only the coarsening
+  const int nb = colored || many ? 0 : g->nb_user;
   const int nkeys = kNumTiers * nb;
   const int64_t nold = (int64_t)kNumTiers * g->nbatches;
   *unsupported = true;
   const int64_t nv = g->nv, ne = g->ne;
-  if (nv < 1 || nv > kStepMaxEdges || ne > kStepMaxEdges || nkeys > kStepKeys || g->gid || g->host_edges ||
-      !loop_plan_fits(g, std::max(nb, 1)) || (coarsen && (!g->loop_plan || !g->bins_valid)))
+  if (nv < 1 || nv > kStepMaxEdges || ne > kStepMaxEdges || nkeys > kStepKeys || g->host_edges)
+    return NIDO_OK;
+  if (many ? !coarsen
+           : !loop_plan_fits(g, std::max(nb, 1)) || (coarsen && (!g->loop_plan || !g->bins_valid)))
     return NIDO_OK;
   StepArgs A;
   memset(&A, 0, sizeof(A));
@@ -632,6 +660,12 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
   A.toff = A.cuts + nb + 1;
   A.tier_off = tier;
   A.coarsen = coarsen;
+  A.setup = !many;
+  if (many) {
+    A.gbase = g->gbase;
+    A.gbase2 = g->gbase2;
+    A.ng = g->ngraphs;
+  }
   A.ordered = !g->int_weights;
   if (coarsen) {
     int64_t slots = 64;
@@ -657,7 +691,8 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
     A.coff = g->off2;
     A.cadj = g->adj2;
     A.cw = g->w2;
-    NIDO_CUDA_TRY(cudaMemcpyAsync(tier, g->tier_off.data(), sizeof(int64_t) * (nold + 1), cudaMemcpyHostToDevice, s));
+    if (!many)
+      NIDO_CUDA_TRY(cudaMemcpyAsync(tier, g->tier_off.data(), sizeof(int64_t) * (nold + 1), cudaMemcpyHostToDevice, s));
   }
   A.err = reinterpret_cast<unsigned long long*>(g->dcount + 1);
   A.warp = g->cfg.warp_max;
@@ -693,6 +728,10 @@ int step(nido_graph_s* g, bool coarsen, int* done, bool* unsupported) {
     g->coarsened = true;
     g->nv = o.nvp;
     g->ne = o.nep;
+  }
+  if (many) {
+    g->bins_valid = false;
+    return NIDO_OK;
   }
   g->m = o.m;
   // where the separate stages look for them
