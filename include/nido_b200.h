@@ -66,14 +66,15 @@ typedef struct {
                         when tau_phase_set, otherwise tau (the reference's
                         three-argument LouvainGPU) */
   int32_t tau_phase_set;
-  int32_t host_loop; /* who drives each phase's iteration loop.  2: the device,
-                        one CUDA graph per phase with a conditional while node,
-                        read back once per phase; 1 or 0 (default): the host,
-                        one Q readback per iteration, as the reference does.
-                        Measured on B200 (driver 580) the host loop is the
-                        faster: building the loop graphs costs more than the
-                        round trips they save, for small and large graphs and
-                        for graph sets alike */
+  int32_t host_loop; /* who drives each phase's iteration loop.  0 (default):
+                        small phases (at most 4 Mi edges, or 1 Mi a batch) run
+                        as one persistent kernel with one readback a phase, and
+                        coarsen in one kernel; larger ones are driven from the
+                        host, one Q readback per iteration.  1: the host always,
+                        as the reference does.  2: one CUDA graph per phase with
+                        a conditional while node, read back once per phase
+                        (building the graphs costs more than the round trips
+                        they save on B200 with driver 580) */
   int32_t color_batches; /* 1: conflict-free batches instead of the -b cuts:
                         every phase colours its graph (Jones-Plassmann-Luby,
                         seed 1) and sweeps the colour classes in colour order,
