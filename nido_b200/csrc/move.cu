@@ -6,10 +6,12 @@
 // neighbour-community weights e_vc are accumulated on chip:
 //   degree <= 32       a group of 4/8/16/32 lanes holds one edge per lane;
 //                      equal communities are found with __match_any_sync and
-//                      their weights folded in edge order (registers only)
-//   degree <= warp_max one warp, open-addressing hash in shared memory
-//   degree <= cta_max  one CTA, hash in shared memory
-//   larger             one CTA, hash in an L2-resident global-memory slab
+//                      their weights folded (registers only)
+//   degree <= 192      one warp, open-addressing table in shared memory
+//   degree <= 12288    one CTA of 128 to 1024 threads, table in shared memory
+//   larger             many CTAs, tables in L2-resident global memory
+// The device code is in move_core.cuh and hub_core.cuh, the kernels of the
+// tiers below the hubs in move_tiers.cuh.
 // Gains and the final decision use the reference's operation order
 // (graph_cuda.cu:1505-1506, 1530-1533):
 //   gain_c = (e_vc - ki*a_c/(2m)) / m,  self = (e_own - ki*(a_own-ki)/(2m)) / m,

@@ -225,9 +225,10 @@ __global__ void __launch_bounds__(kLoopThreads, 4) k_phase_loop(const __grid_con
         }
         // A vertex of 100 to 190 edges takes a warp eight to ten microseconds,
         // chunk after chunk, and a CTA three: while the batch has at most two of
-        // them a block, CTAs take the warp tier as well.
+        // them a block, CTAs take the warp tier as well.  Integer phases only: a
+        // CTA's FP64 sums are atomic, a warp's are in a fixed order.
         const int64_t nwarp = to[(int64_t)kTierWarp * nb + 1] - to[(int64_t)kTierWarp * nb];
-        const int lowest = nwarp <= 2 * (int64_t)gridDim.x ? kTierWarp : kTierCtaS;
+        const int lowest = kInts && nwarp <= 2 * (int64_t)gridDim.x ? kTierWarp : kTierCtaS;
         for (int tier = kTierCtaL; tier >= lowest; --tier) {
           const int64_t l0 = to[(int64_t)tier * nb], n = to[(int64_t)tier * nb + 1] - l0;
           int64_t i = (int64_t)blockIdx.x - rot;

@@ -12,8 +12,8 @@
 // ascending member order, one coarse vertex after the other; a bitmap of the
 // first positions then ranks every entry by a popcount prefix, which is its
 // place in the coarse CSR in the reference's first-occurrence order.  Equal
-// neighbours of a 32-edge chunk are folded in edge order before they are
-// added; across chunks the adds are atomic (exact for integer weights, as in
+// neighbours of a 32-edge chunk are folded before they are added; across
+// chunks the adds are atomic (exact for integer weights, as in
 // the CTA tiers of coarsen.cu).  In FP64 phases the weights of coarse vertices
 // of at most 1024 member edges are added in list order instead: every edge notes
 // its entry and weight at its list position, and a warp walks the list.  Up to
