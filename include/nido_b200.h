@@ -67,7 +67,7 @@ typedef struct {
                         three-argument LouvainGPU) */
   int32_t tau_phase_set;
   int32_t host_loop; /* who drives each phase's iteration loop.  0 (default):
-                        small phases (at most 4 Mi edges, or 1 Mi a batch) run
+                        small phases (at most 9 Mi edges, or 1 Mi a batch) run
                         as one persistent kernel with one readback a phase, and
                         coarsen in one kernel; larger ones are driven from the
                         host, one Q readback per iteration.  1: the host always,

@@ -663,6 +663,7 @@ extern "C" int nido_batch_run(nido_batch B, const nido_params* p, int64_t* out_c
   if (p->tie_mode != NIDO_TIE_SMALLEST_ID && p->tie_mode != NIDO_TIE_NIDO)
     return nido_set_error(NIDO_E_INVALID, "unknown tie mode %d", p->tie_mode);
   NIDO_CUDA_TRY(cudaSetDevice(g->ctx->device));
+  set_plan_tie(g, p->tie_mode);
   cudaStream_t s = g->ctx->stream;
   nido_run_stats st;
   memset(&st, 0, sizeof(st));

@@ -1050,6 +1050,7 @@ extern "C" int nido_run(nido_graph g, const nido_params* p, int64_t* out_comm, n
   if (p->tie_mode != NIDO_TIE_SMALLEST_ID && p->tie_mode != NIDO_TIE_NIDO)
     return nido_set_error(NIDO_E_INVALID, "unknown tie mode %d", p->tie_mode);
   NIDO_CUDA_TRY(cudaSetDevice(g->ctx->device));
+  nido::set_plan_tie(g, p->tie_mode);
   nido_run_stats st;
   memset(&st, 0, sizeof(st));
   cudaStream_t s = g->ctx->stream;

@@ -215,6 +215,7 @@ struct nido_graph_s {
   std::vector<int64_t> tier_off; // host: nbatches*kNumTiers+1 offsets into perm
   bool bins_valid = false;
   int64_t plan_ne = -1;          // many graphs: edges of the listed graphs (-1: ne)
+  bool plan_tie = false;         // the lists are for a run under the reference's tie rule
   bool loop_plan = false;        // the tier lists are cut for the persistent phase loop
   int64_t max_degree = 0;
   TierConfig cfg;
@@ -317,11 +318,17 @@ int device_phase_loop(nido_graph_s* g, int tie, double tau, int64_t max_iter, bo
 // Phases of at most kLoopMaxEdges edges, or kLoopMaxBatchEdges a batch, run on it by
 // default.  A batch of a few hundred thousand edges is launch-bound on the
 // per-tier kernels: 22.8 M edges in 32 batches take 1.4 ms a sweep on them and
-// 0.95 ms here, 2.0 M edges in one batch 0.16 and 0.10 ms.  The per-tier
-// kernels keep more warps resident and win above: 57.9 M edges in 32 batches 3.0
-// against 3.3 ms, 7.6 M in two batches (reference tie rule) 0.5 against 0.7 ms.
-constexpr int64_t kLoopMaxEdges = (int64_t)4 << 20;
+// 0.95 ms here, and whole runs of R-MAT of 8.9 M edges in two batches 38.0 (integer
+// weights) and 16.9 ms (uniform) against 34.5 and 15.8 ms.  The per-tier kernels
+// keep more warps resident and win above: SBM of 11.0 M edges 14.2 against 14.8
+// ms, R-MAT of 14.7 M 38.6 against 39.8 ms.  Under the reference's tie rule they win
+// sooner, as one block evaluates a hub: 22.5 against 27.6 ms at 7.6 M.
+constexpr int64_t kLoopMaxEdges = (int64_t)9 << 20;
+constexpr int64_t kLoopMaxEdgesTie = (int64_t)4 << 20;
 constexpr int64_t kLoopMaxBatchEdges = (int64_t)1 << 20;
+// the run's tie rule, which moves the bound: lists cut for the other rule are
+// built again when they would differ (phase.cu)
+void set_plan_tie(nido_graph_s* g, int tie);
 bool loop_plan_fits(const nido_graph_s* g, int nb);  // the phase (nb batches) is one of those (phase.cu)
 struct LoopGraphs {  // many graphs: the listed graphs and their loop state (device)
   const int32_t* gl;

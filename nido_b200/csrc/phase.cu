@@ -580,10 +580,19 @@ int launch_modularity_dev(nido_graph_s* g) {
 bool loop_plan_fits(const nido_graph_s* g, int nb) {
   const TierConfig d;
   const int64_t ne = g->gid && g->plan_ne >= 0 ? g->plan_ne : g->ne;
-  return !g->host_edges && (ne <= kLoopMaxEdges || ne / nb <= kLoopMaxBatchEdges) && g->cfg.warp_max == d.warp_max &&
+  return !g->host_edges && (ne <= (g->plan_tie ? kLoopMaxEdgesTie : kLoopMaxEdges) || ne / nb <= kLoopMaxBatchEdges) && g->cfg.warp_max == d.warp_max &&
          g->cfg.ctas_max == d.ctas_max && g->cfg.ctam_max == d.ctam_max && g->cfg.ctal_max == d.ctal_max &&
          g->cfg.ctax_max == d.ctax_max && !g->cfg.hub_clusters && !g->cfg.staged_edges &&
          g->cfg.hub_wave_slots == d.hub_wave_slots;
+}
+
+void set_plan_tie(nido_graph_s* g, int tie) {
+  const bool t = tie == NIDO_TIE_NIDO;
+  if (t == g->plan_tie) return;
+  const int nb = std::max(g->nbatches, 1);
+  const bool before = loop_plan_fits(g, nb);
+  g->plan_tie = t;
+  if (loop_plan_fits(g, nb) != before) g->bins_valid = false;
 }
 
 int build_batches(nido_graph_s* g) {
